@@ -91,6 +91,7 @@ struct lf_scene
     int* d_parent = nullptr;
     int* d_leafOfTri = nullptr;     // reference leaf of every triangle
     int* d_leafOfInst = nullptr;    // reference leaf of every instance
+    int* d_instOfTri = nullptr;     // instance of the triangles merged into the instance level
     float boundsLo[3] = {0, 0, 0}, boundsHi[3] = {0, 0, 0};   // instance-level root box
 };
 

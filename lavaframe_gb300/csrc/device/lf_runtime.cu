@@ -305,31 +305,79 @@ lf_status encode_level(lf_ctx* c, const RefNode* nodes, int numNodes, int start,
 // Every wide node holds up to four reference nodes as children: starting from a reference
 // inner node's two children, the inner child with the largest box surface area is replaced by
 // its two children until four children are reached or only leaves remain. Leaves keep the
-// binary encoding's codes; every child slot carries the reference node's own box and index.
+// binary encoding's codes (instances with kWideInstLeaf set); every child slot carries the
+// reference node's own box and index.
+//
+// An instance whose inverse transform is the identity and whose mesh no other instance uses is
+// merged into the instance level: its leaf counts as the mesh's root, so nodes may collapse
+// across the two levels and its triangles are leaves of the instance level's tree. The object
+// ray of such an instance is the world ray (the transform's products and sums reproduce every
+// finite component, and a zero origin component as +0), so the boxes and triangles tested give
+// the same values, and a triangle's leaf passes only if the instance's box does, because
+// inlinable() asks for the mesh root's child boxes to lie inside it.
 struct WideBuilder
 {
     const RefNode* nodes = nullptr;
     int numNodes = 0, numTris = 0, numInstances = 0;
     std::vector<float4> recs;
-    std::vector<int> map;   // reference inner node -> wide record it heads
+    std::vector<int> map;         // reference inner node -> wide record it heads
+    std::vector<int> inlineRoot;  // per instance: the mesh root merged into the instance level, -1 if none
+    std::vector<int> instOfTri;   // instance of the triangles of merged meshes, -1 otherwise
 };
 
-bool ref_leaf_code(const RefNode& n, bool meshLevel, int numTris, int numInstances, int* code)
+// A child of a wide node: the reference node whose box it has and the one whose contents it
+// stands for (they differ for a merged instance: its leaf's box, its mesh's root).
+struct WideItem
 {
+    int box, node;
+    bool mesh;   // the contents are on the mesh level
+    int inst;    // merged instance the contents belong to, -1 if none
+};
+
+bool ref_leaf_code(WideBuilder& B, const WideItem& it, int* code)
+{
+    const RefNode& n = B.nodes[it.node];
     const int z = (int)n.lr[2];
-    if (meshLevel)
+    if (it.mesh)
     {
         if (z <= 0) return false;
         const int first = (int)n.lr[0], cnt = (int)n.lr[1];
-        if (first < 0 || cnt < 0 || cnt > 3 || first + cnt > numTris) return false;
+        if (first < 0 || cnt < 0 || cnt > 3 || first + cnt > B.numTris) return false;
+        if (it.inst >= 0) std::fill(B.instOfTri.begin() + first, B.instOfTri.begin() + first + cnt, it.inst);
         *code = ~((first << 2) | cnt);
     }
     else
     {
         if (z >= 0) return false;
         const int inst = -z - 1;
-        if (inst >= numInstances) return false;
-        *code = ~inst;
+        if (inst >= B.numInstances) return false;
+        *code = ~(inst | kWideInstLeaf);
+    }
+    return true;
+}
+
+WideItem wide_item(const WideBuilder& B, int k, bool mesh, int inst)
+{
+    const int z = (int)B.nodes[k].lr[2];
+    if (!mesh && z < 0 && -z - 1 < B.numInstances && B.inlineRoot[-z - 1] >= 0)
+        return {k, B.inlineRoot[-z - 1], true, -z - 1};
+    return {k, k, mesh, inst};
+}
+
+// Whether the mesh at reference node `root` can be merged into the instance level in the place of the
+// instance leaf `leaf`: the boxes of the root's children lie inside the leaf's box.
+bool inlinable(const WideBuilder& B, int leaf, int root)
+{
+    if (root < 0 || root >= B.numNodes) return false;
+    const RefNode &L = B.nodes[leaf], &R = B.nodes[root];
+    if ((int)R.lr[2] != 0) return true;   // a leaf is tested without a box of its own
+    for (int k = 0; k < 2; ++k)
+    {
+        const int ci = (int)R.lr[k];
+        if (ci < 0 || ci >= B.numNodes) return false;
+        const RefNode& C = B.nodes[ci];
+        for (int a = 0; a < 3; ++a)
+            if (!(C.bmin[a] >= L.bmin[a] && C.bmax[a] <= L.bmax[a])) return false;
     }
     return true;
 }
@@ -343,47 +391,55 @@ float box_area(const RefNode& n)
 lf_status wide_level(lf_ctx* c, WideBuilder& B, int start, bool meshLevel, int* rootCode)
 {
     if (start < 0 || start >= B.numNodes) return fail(c, LF_ERR_INVALID, "node index out of range");
-    const RefNode& r = B.nodes[start];
-    if ((int)r.lr[2] != 0)
+    const WideItem top = wide_item(B, start, meshLevel, -1);
+    auto inner = [&](const WideItem& i) { return (int)B.nodes[i.node].lr[2] == 0; };
+    if (!inner(top))
     {
-        if (!ref_leaf_code(r, meshLevel, B.numTris, B.numInstances, rootCode))
+        if (!ref_leaf_code(B, top, rootCode))
             return fail(c, LF_ERR_INVALID, "bad leaf node " + std::to_string(start));
         return LF_OK;
     }
-    if (B.map[start] >= 0)
+    if (B.map[top.node] >= 0)
     {
-        *rootCode = B.map[start];
+        *rootCode = B.map[top.node];
         return LF_OK;
     }
-    auto inner = [&](int i) { return (int)B.nodes[i].lr[2] == 0; };
-    B.map[start] = (int)(B.recs.size() / kWideF4);
+    B.map[top.node] = (int)(B.recs.size() / kWideF4);
     B.recs.resize(B.recs.size() + kWideF4);
-    std::vector<int> stack{start};
+    std::vector<WideItem> stack{top};
     while (!stack.empty())
     {
-        const int ref = stack.back();
+        const WideItem ref = stack.back();
         stack.pop_back();
-        const int rec = B.map[ref];
-        std::vector<int> kids{(int)B.nodes[ref].lr[0], (int)B.nodes[ref].lr[1]};
-        for (int k : kids)
-            if (k < 0 || k >= B.numNodes) return fail(c, LF_ERR_INVALID, "child index out of range");
-        while ((int)kids.size() < kWide)
+        const int rec = B.map[ref.node];
+        WideItem kids[kWide];
+        int nk = 0;
+        // the two children of an inner node as items at positions at, at + 1 (the items from at + 1
+        // on move up by one)
+        auto put_children = [&](const WideItem& x, int at) {
+            const int xl = (int)B.nodes[x.node].lr[0], xr = (int)B.nodes[x.node].lr[1];
+            if (xl < 0 || xl >= B.numNodes || xr < 0 || xr >= B.numNodes) return false;
+            for (int k = nk; k > at + 1; --k) kids[k] = kids[k - 1];
+            kids[at] = wide_item(B, xl, x.mesh, x.inst);
+            kids[at + 1] = wide_item(B, xr, x.mesh, x.inst);
+            return true;
+        };
+        if (!put_children(ref, 0)) return fail(c, LF_ERR_INVALID, "child index out of range");
+        nk = 2;
+        while (nk < kWide)
         {
             int best = -1;
             float area = -1.f;
-            for (int k = 0; k < (int)kids.size(); ++k)
-                if (inner(kids[k]) && box_area(B.nodes[kids[k]]) > area)
+            for (int k = 0; k < nk; ++k)
+                if (inner(kids[k]) && box_area(B.nodes[kids[k].box]) > area)
                 {
-                    area = box_area(B.nodes[kids[k]]);
+                    area = box_area(B.nodes[kids[k].box]);
                     best = k;
                 }
             if (best < 0) break;
-            const int x = kids[best];
-            const int xl = (int)B.nodes[x].lr[0], xr = (int)B.nodes[x].lr[1];
-            if (xl < 0 || xl >= B.numNodes || xr < 0 || xr >= B.numNodes)
-                return fail(c, LF_ERR_INVALID, "child index out of range");
-            kids[best] = xl;
-            kids.insert(kids.begin() + best + 1, xr);
+            const WideItem x = kids[best];
+            if (!put_children(x, best)) return fail(c, LF_ERR_INVALID, "child index out of range");
+            ++nk;
         }
         float f[8][kWide];
         for (int j = 0; j < kWide; ++j)
@@ -393,26 +449,27 @@ lf_status wide_level(lf_ctx* c, WideBuilder& B, int start, bool meshLevel, int* 
             // (wide_slabs) its entry is +inf and its exit -inf for every ray, so no test passes
             const float inf = std::numeric_limits<float>::infinity();
             float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
-            if (j < (int)kids.size())
+            if (j < nk)
             {
-                const int k = kids[j];
-                const RefNode& n = B.nodes[k];
+                const WideItem& k = kids[j];
+                const RefNode& n = B.nodes[k.box];
                 for (int a = 0; a < 3; ++a)
                 {
                     lo[a] = n.bmin[a];
                     hi[a] = n.bmax[a];
                 }
-                refIdx = k;
+                refIdx = k.box;
                 if (inner(k))
                 {
-                    if (B.map[k] >= 0) return fail(c, LF_ERR_INVALID, "node referenced twice: " + std::to_string(k));
-                    B.map[k] = (int)(B.recs.size() / kWideF4);
+                    if (B.map[k.node] >= 0)
+                        return fail(c, LF_ERR_INVALID, "node referenced twice: " + std::to_string(k.node));
+                    B.map[k.node] = (int)(B.recs.size() / kWideF4);
                     B.recs.resize(B.recs.size() + kWideF4);
-                    code = B.map[k];
+                    code = B.map[k.node];
                     stack.push_back(k);
                 }
-                else if (!ref_leaf_code(n, meshLevel, B.numTris, B.numInstances, &code))
-                    return fail(c, LF_ERR_INVALID, "bad leaf node " + std::to_string(k));
+                else if (!ref_leaf_code(B, k, &code))
+                    return fail(c, LF_ERR_INVALID, "bad leaf node " + std::to_string(k.node));
             }
             f[0][j] = lo[0];
             f[1][j] = hi[0];
@@ -428,7 +485,7 @@ lf_status wide_level(lf_ctx* c, WideBuilder& B, int start, bool meshLevel, int* 
             for (int h4 = 0; h4 < kWide / 4; ++h4)
                 o[g * (kWide / 4) + h4] = make_float4(f[g][h4 * 4], f[g][h4 * 4 + 1], f[g][h4 * 4 + 2], f[g][h4 * 4 + 3]);
     }
-    *rootCode = B.map[start];
+    *rootCode = B.map[top.node];
     return LF_OK;
 }
 
@@ -437,7 +494,7 @@ lf_status wide_level(lf_ctx* c, WideBuilder& B, int start, bool meshLevel, int* 
 // reference leaf that holds each triangle and each instance (tie resolution only).
 lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, std::vector<float4>& inst,
                       std::vector<float4>& wrecs, std::vector<int>& parent, std::vector<int>& leafOfTri,
-                      std::vector<int>& leafOfInst, int* wroot)
+                      std::vector<int>& leafOfInst, std::vector<int>& instOfTri, int* wroot)
 {
     WideBuilder B;
     B.nodes = nodes;
@@ -445,7 +502,10 @@ lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, s
     B.numTris = v->num_tris;
     B.numInstances = v->num_instances;
     B.map.assign(v->num_nodes, -1);
-    std::vector<int> instRoot(v->num_instances, -1);
+    B.inlineRoot.assign(v->num_instances, -1);
+    B.instOfTri.assign(std::max(v->num_tris, 1), -1);
+    std::vector<int> instRoot(v->num_instances, -1), instLeaf(v->num_instances, -1);
+    std::vector<unsigned char> rootUses(v->num_nodes, 0);   // instances of a mesh root, up to 2
     std::vector<int> stack{v->top_level_index};
     while (!stack.empty())
     {
@@ -454,17 +514,30 @@ lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, s
         const RefNode& n = nodes[ref];
         const int z = (int)n.lr[2];
         if (z < 0)
-            instRoot[-z - 1] = (int)n.lr[0];
+        {
+            const int root = (int)n.lr[0];
+            instRoot[-z - 1] = root;
+            instLeaf[-z - 1] = ref;
+            if (root >= 0 && root < v->num_nodes && rootUses[root] < 2) ++rootUses[root];
+        }
         else if (z == 0)
         {
             stack.push_back((int)n.lr[1]);
             stack.push_back((int)n.lr[0]);
         }
     }
+    // instances merged into the instance level: identity inverse (bit for bit), a mesh of their own
+    const float4 identity[3] = {make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0)};
+    for (int i = 0; i < v->num_instances; ++i)
+        if (instRoot[i] >= 0 && instRoot[i] < v->num_nodes && rootUses[instRoot[i]] == 1 &&
+            std::memcmp(&inst[(size_t)i * 4], identity, sizeof identity) == 0 && inlinable(B, instLeaf[i], instRoot[i]))
+            B.inlineRoot[i] = instRoot[i];
     for (int i = 0; i < v->num_instances; ++i)
     {
         int code = ~0, rootRef = -1;
-        if (instRoot[i] >= 0)
+        if (B.inlineRoot[i] >= 0)
+            rootRef = instRoot[i];   // reached through the instance level only
+        else if (instRoot[i] >= 0)
         {
             lf_status st = wide_level(c, B, instRoot[i], true, &code);
             if (st != LF_OK) return st;
@@ -479,6 +552,7 @@ lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, s
     lf_status st = wide_level(c, B, v->top_level_index, false, wroot);
     if (st != LF_OK) return st;
     wrecs.swap(B.recs);
+    instOfTri.swap(B.instOfTri);
     parent.assign(v->num_nodes, -1);
     leafOfTri.assign(std::max(v->num_tris, 1), -1);
     leafOfInst.assign(std::max(v->num_instances, 1), -1);
@@ -636,9 +710,9 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     lf_status st = encode_instances(c, v, nodes, recs, map, inst, sinst, &tlasRoot);
     if (st != LF_OK) return st;
     std::vector<float4> wrecs;
-    std::vector<int> parent, leafOfTri, leafOfInst;
+    std::vector<int> parent, leafOfTri, leafOfInst, instOfTri;
     int wroot = 0;
-    st = encode_wide(c, v, nodes, inst, wrecs, parent, leafOfTri, leafOfInst, &wroot);
+    st = encode_wide(c, v, nodes, inst, wrecs, parent, leafOfTri, leafOfInst, instOfTri, &wroot);
     if (st != LF_OK) return st;
     // room for a re-encoded instance level after instance updates (at most one wide node per
     // inner node of the instance tree)
@@ -694,12 +768,13 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     float4* d_wide = nullptr;
     float* d_refNodes = nullptr;
     int* d_parent = nullptr;
-    int *d_leafOfTri = nullptr, *d_leafOfInst = nullptr;
+    int *d_leafOfTri = nullptr, *d_leafOfInst = nullptr, *d_instOfTri = nullptr;
     A(&d_wide, wideCap * kWideF4);
     A(&d_refNodes, (size_t)v->num_nodes * 9);
     A(&d_parent, (size_t)v->num_nodes);
     A(&d_leafOfTri, leafOfTri.size());
     A(&d_leafOfInst, leafOfInst.size());
+    A(&d_instOfTri, instOfTri.size());
     float* d_env = nullptr;
     float2 *d_marg = nullptr, *d_cond = nullptr;
     uint8_t* d_tex = nullptr;
@@ -734,6 +809,7 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     H2D(d_parent, parent.data(), parent.size() * sizeof(int));
     H2D(d_leafOfTri, leafOfTri.data(), leafOfTri.size() * sizeof(int));
     H2D(d_leafOfInst, leafOfInst.data(), leafOfInst.size() * sizeof(int));
+    H2D(d_instOfTri, instOfTri.data(), instOfTri.size() * sizeof(int));
     if (hasEnv)
     {
         H2D(d_env, v->env_rgb, (size_t)v->env_width * v->env_height * 3 * sizeof(float));
@@ -766,6 +842,7 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     S.trav.refParent = d_parent;
     S.trav.leafOfTri = d_leafOfTri;
     S.trav.leafOfInst = d_leafOfInst;
+    S.trav.instOfTri = d_instOfTri;
     S.vertIndices = d_vidx;
     S.vertices = d_verts;
     S.normals = d_norms;
@@ -801,6 +878,7 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     sc->d_parent = d_parent;
     sc->d_leafOfTri = d_leafOfTri;
     sc->d_leafOfInst = d_leafOfInst;
+    sc->d_instOfTri = d_instOfTri;
     sc->d_instances = d_inst;
     sc->d_sinst = d_sinst;
     sc->d_materials = d_mats;
@@ -831,12 +909,30 @@ lf_status lf_scene_update_instances(lf_scene* sc, const lf_scene_view* v)
     if (st != LF_OK) return st;
     if (recs.size() / 4 > sc->nodeCapacity) return fail(c, LF_ERR_INVALID, "instance update grew the node array");
     std::vector<float4> wrecs;
-    std::vector<int> parent, leafOfTri, leafOfInst;
+    std::vector<int> parent, leafOfTri, leafOfInst, instOfTri;
     int wroot = 0;
-    st = encode_wide(c, v, nodes, inst, wrecs, parent, leafOfTri, leafOfInst, &wroot);
+    st = encode_wide(c, v, nodes, inst, wrecs, parent, leafOfTri, leafOfInst, instOfTri, &wroot);
     if (st != LF_OK) return st;
-    if (wrecs.size() / kWideF4 > sc->wideCapacity) return fail(c, LF_ERR_INVALID, "instance update grew the wide tree");
     cudaError_t e = cudaStreamSynchronize(c->stream);
+    const size_t wideNodes = wrecs.size() / kWideF4;
+    if (e == cudaSuccess && wideNodes > sc->wideCapacity)
+    {
+        // instances that stopped (or started) being merged changed how nodes collapse: a larger
+        // array takes the old one's place
+        float4* grown = nullptr;
+        e = cudaMalloc((void**)&grown, wideNodes * kWideF4 * sizeof(float4));
+        if (e == cudaSuccess)
+        {
+            std::replace(sc->allocs.begin(), sc->allocs.end(), (void*)sc->d_wide, (void*)grown);
+            cudaFree(sc->d_wide);
+            sc->bytes += (wideNodes - sc->wideCapacity) * kWideF4 * sizeof(float4);
+            sc->wideCapacity = wideNodes;
+            sc->d_wide = grown;
+            sc->view.trav.wnodes = grown;
+        }
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpy(sc->d_instOfTri, instOfTri.data(), instOfTri.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(sc->d_wide, wrecs.data(), wrecs.size() * sizeof(float4), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(sc->d_refNodes, v->nodes, (size_t)v->num_nodes * 9 * sizeof(float), cudaMemcpyHostToDevice);
