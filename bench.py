@@ -808,8 +808,8 @@ def main():
             "cpu_baseline": {"value": cpu_v, "unit": "Grays/s", "cores": cores, "kind": "port",
                              "sample": f"{sample} of the 2^{args.rays_log2} rays, {cpu_dt:.1f} s"},
             "clocks": clocks,
-            # per binned query: ray_keys, the three bin-scan kernels, ray_scatter, traversal
-            "gpu_launches": args.steps * 6,
+            # per binned query: ray_keys, bin scan, ray_scatter, traversal
+            "gpu_launches": args.steps * 4,
             "extra": extra,
         }
         print(json.dumps(line), flush=True)

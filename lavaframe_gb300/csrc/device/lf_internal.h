@@ -29,7 +29,10 @@ struct lf_ctx
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::string err;
-    uint32_t* d_status = nullptr;
+    // status word of the kernels: in mapped page-locked memory, so that reading it after a
+    // synchronisation needs no copy (the kernels only write it when something went wrong)
+    volatile uint32_t* h_status = nullptr;
+    uint32_t* d_status = nullptr;         // its device address
     unsigned long long* d_stats = nullptr;   // [3] traversal counters
     uint32_t devErrors = 0;
     uint64_t lastStats[3] = {0, 0, 0};
@@ -59,7 +62,9 @@ struct lf_ctx
     int* binPerm = nullptr;
     size_t binCap = 0;
     uint32_t* binHist = nullptr;
-    unsigned long long* binNext = nullptr;
+    unsigned long long* binNext = nullptr;   // fetch counter and blocks done, zero between launches
+    char* stage = nullptr;                   // page-locked staging of small host queries
+    char* d_stage = nullptr;                 // its device address
     lfrt::EngineHost* engine = nullptr;   // multi-job engine, created on first use
     // traversal-kernel timer of the binned ray queries: one event pair per launch while on
     bool kernelTimer = false;
@@ -168,13 +173,11 @@ inline lf_status check_device(lf_ctx* c)
 {
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "stream synchronize");
-    uint32_t bits = 0;
-    e = cudaMemcpy(&bits, c->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(c, e, "status readback");
+    const uint32_t bits = *c->h_status;
     if (bits)
     {
         c->devErrors |= bits;
-        cudaMemset(c->d_status, 0, sizeof(uint32_t));
+        *c->h_status = 0;
         return fail(c, LF_ERR_DEVICE, "device error bits 0x" + std::to_string(bits));
     }
     return LF_OK;

@@ -29,13 +29,14 @@ lf_status lf_ctx_create(int32_t device, lf_ctx** out)
     lf_ctx* c = new lf_ctx;
     c->device = device;
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaMalloc((void**)&c->d_status, sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaHostAlloc((void**)&c->h_status, sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
+        (e = cudaHostGetDevicePointer((void**)&c->d_status, (void*)c->h_status, 0)) != cudaSuccess ||
         (e = cudaMalloc((void**)&c->d_stats, 3 * sizeof(unsigned long long))) != cudaSuccess)
     {
         delete c;
         return e == cudaErrorMemoryAllocation ? LF_ERR_OOM : LF_ERR_CUDA;
     }
-    cudaMemset(c->d_status, 0, sizeof(uint32_t));
+    *c->h_status = 0;
     cudaMemset(c->d_stats, 0, 3 * sizeof(unsigned long long));
     *out = c;
     return LF_OK;
@@ -48,7 +49,8 @@ void lf_ctx_destroy(lf_ctx* c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     engine_destroy(c->engine);
     c->engine = nullptr;
-    cudaFree(c->d_status);
+    cudaFreeHost((void*)c->h_status);
+    cudaFreeHost(c->stage);
     cudaFree(c->d_stats);
     cudaFree(c->scratchRays);
     cudaFree(c->scratchOut);
@@ -993,13 +995,20 @@ size_t lf_scene_device_bytes(const lf_scene* sc) { return sc ? sc->bytes : 0; }
 
 namespace
 {
-// Grows the binning scratch (keys, permutation, bin counters, fetch counter) of a context.
-lf_status ensure_bin_scratch(lf_ctx* c, long long n)
+// Scratch of the ray queries: the fetch counters, and for a binned query of n rays the bins, keys
+// and permutation.
+lf_status ensure_bin_scratch(lf_ctx* c, long long n, bool binned)
 {
+    if (!c->binNext)
+    {
+        cudaError_t e = cudaMalloc((void**)&c->binNext, 2 * sizeof(unsigned long long));
+        if (e == cudaSuccess) e = cudaMemsetAsync(c->binNext, 0, 2 * sizeof(unsigned long long), c->stream);
+        if (e != cudaSuccess) return cuda_fail(c, e, "binning scratch");
+    }
+    if (!binned) return LF_OK;
     if (!c->binHist)
     {
         cudaError_t e = cudaMalloc((void**)&c->binHist, sizeof(uint32_t) * (size_t)trace_bins());
-        if (e == cudaSuccess) e = cudaMalloc((void**)&c->binNext, sizeof(unsigned long long));
         if (e != cudaSuccess) return cuda_fail(c, e, "binning scratch");
     }
     if ((size_t)n > c->binCap)
@@ -1048,12 +1057,13 @@ lf_status lf_trace_closest_device(lf_ctx* c, lf_scene* sc, const void* d_rays, i
     int e;
     if (!stats && !(flags & LF_TRACE_SIMPLE))
     {
-        lf_status bs = ensure_bin_scratch(c, n);
+        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, false);
+        lf_status bs = ensure_bin_scratch(c, n, binned);
         if (bs != LF_OK) return bs;
         cudaEvent_t k0, k1;
         kernel_timer_pair(c, &k0, &k1);
         e = launch_trace_binned(sc->view.trav, (const float4*)d_rays, n, d_hits, false, (flags & LF_TRACE_LIGHTS) ? 1 : 0,
-                                sc->boundsLo, sc->boundsHi, !(flags & LF_TRACE_UNSORTED), c->binKeys, c->binHist,
+                                sc->boundsLo, sc->boundsHi, binned, c->binKeys, c->binHist,
                                 c->binPerm, c->binNext, c->d_status, c->stream, k0, k1);
     }
     else
@@ -1074,12 +1084,13 @@ lf_status lf_trace_any_device(lf_ctx* c, lf_scene* sc, const void* d_rays, int64
     int e;
     if (!stats && !(flags & LF_TRACE_SIMPLE))
     {
-        lf_status bs = ensure_bin_scratch(c, n);
+        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, true);
+        lf_status bs = ensure_bin_scratch(c, n, binned);
         if (bs != LF_OK) return bs;
         cudaEvent_t k0, k1;
         kernel_timer_pair(c, &k0, &k1);
         e = launch_trace_binned(sc->view.trav, (const float4*)d_rays, n, d_occ, true, (flags & LF_TRACE_LIGHTS) ? 1 : 0,
-                                sc->boundsLo, sc->boundsHi, !(flags & LF_TRACE_UNSORTED), c->binKeys, c->binHist,
+                                sc->boundsLo, sc->boundsHi, binned, c->binKeys, c->binHist,
                                 c->binPerm, c->binNext, c->d_status, c->stream, k0, k1);
     }
     else
@@ -1131,6 +1142,30 @@ char* mapped_range(const lf_ctx* c, const void* p, size_t bytes)
     return nullptr;
 }
 
+constexpr size_t kStageBytes = size_t(1) << 18;
+
+// The context's page-locked staging block, mapped for the kernels; false when there is none.
+bool ensure_stage(lf_ctx* c)
+{
+    if (c->stage) return true;
+    if (cudaHostAlloc((void**)&c->stage, kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&c->d_stage, c->stage, 0) != cudaSuccess)
+    {
+        cudaGetLastError();
+        if (c->stage) cudaFreeHost(c->stage);
+        c->stage = nullptr;
+        return false;
+    }
+    return true;
+}
+
+void read_trace_stats(lf_ctx* c)
+{
+    unsigned long long s[3];
+    cudaMemcpy(s, c->d_stats, sizeof s, cudaMemcpyDeviceToHost);
+    for (int k = 0; k < 3; ++k) c->lastStats[k] = s[k];
+}
+
 // Copies the rays in, traces them and copies the results out, in `host_chunks` pieces: piece k
 // is copied in on copyIn, sorted and traced on the context stream once its copy is done, and
 // copied out on copyOut once traced, so copies of some pieces overlap the tracing of others.
@@ -1155,6 +1190,19 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
         if (err == cudaSuccess) *cap = bytes;
         return err;
     };
+    if ((size_t)n * (32 + outElem) <= kStageBytes && ensure_stage(c))
+    {
+        // small queries: the kernels read the rays from page-locked memory and write the results
+        // there, so that the call is one launch and one wait
+        char* s_out = c->stage + (size_t)n * 32;
+        std::memcpy(c->stage, rays, (size_t)n * 32);
+        lf_status sst = launch(c->d_stage, c->d_stage + (size_t)n * 32, n);
+        const lf_status dst = check_device(c);
+        if (sst == LF_OK) sst = dst;
+        if (sst == LF_OK) std::memcpy(out, s_out, (size_t)n * outElem);
+        if (sst == LF_OK && (flags & LF_TRACE_STATS)) read_trace_stats(c);
+        return sst;
+    }
     char* direct = mapped_range(c, out, (size_t)n * outElem);
     cudaError_t e = ensure(&c->scratchRays, &c->scratchRaysBytes, (size_t)n * 32);
     if (e == cudaSuccess && !direct) e = ensure(&c->scratchOut, &c->scratchOutBytes, (size_t)n * outElem);
@@ -1204,12 +1252,7 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
     }
     if (e == cudaSuccess && st == LF_OK) st = check_device(c);
     else cudaStreamSynchronize(c->stream);   // no copy may still touch the caller's buffers
-    if (e == cudaSuccess && st == LF_OK && (flags & LF_TRACE_STATS))
-    {
-        unsigned long long s[3];
-        cudaMemcpy(s, c->d_stats, sizeof s, cudaMemcpyDeviceToHost);
-        for (int k = 0; k < 3; ++k) c->lastStats[k] = s[k];
-    }
+    if (e == cudaSuccess && st == LF_OK && (flags & LF_TRACE_STATS)) read_trace_stats(c);
     if (e != cudaSuccess) return cuda_fail(c, e, "trace");
     return st;
 }

@@ -2,14 +2,18 @@
 // traversal kernel.
 //
 // Random rays give each lane of a warp its own path through the BVH: few lanes share an
-// instruction and almost every node comes from DRAM. Two measures, neither of which changes
+// instruction and almost every node comes from DRAM. Three measures, none of which changes
 // any per-ray result:
-//  - binning: rays are counting-sorted by a key made of the Morton code of their origin
-//    cell (64^3 cells over the scene box; 16^3 and 32^3 measured 3 % and 1.3 % slower on the
-//    microbench) and their direction octant, so neighbouring lanes start in the same region
-//    heading the same way and share nodes in L1/L2;
-//  - persistent warps with dynamic fetch: warps take rays 32 at a time from a counter in the
-//    binned order, so a warp that finished early takes more work.
+//  - binning: rays of large queries are counting-sorted by a key made of the Morton code of
+//    their origin cell (64^3 cells over the scene box, 32^3 below kFineRays) and their direction
+//    octant, so neighbouring lanes start in the same region heading the same way and share nodes
+//    in L1/L2;
+//  - persistent warps with dynamic fetch: warps take rays from a counter in the binned order, so
+//    a warp that finished early takes more work;
+//  - queries that cannot fill the GPU put fewer rays into a warp (chunk_for): with 32 rays a
+//    warp runs the union of their branches, with few it runs little more than one ray's.
+#include <algorithm>
+
 #include "lf_kernels.h"
 
 namespace lfd
@@ -17,20 +21,29 @@ namespace lfd
 namespace
 {
 constexpr unsigned kFullMask = 0xffffffffu;
-#ifndef LF_TRACE_CELL_BITS
-#define LF_TRACE_CELL_BITS 6
-#endif
-constexpr int kCellBits = LF_TRACE_CELL_BITS;          // cells per axis = 2^kCellBits
-constexpr int kCells = 1 << kCellBits;
-constexpr int kBinBits = 3 * kCellBits + 3;            // origin Morton code + direction octant
-constexpr int kBins = 1 << kBinBits;
+constexpr int kCellBits = 6;                           // most cells per axis = 2^kCellBits
+constexpr int bins_of(int cellBits) { return 1 << (3 * cellBits + 3); }   // origin Morton code + direction octant
 constexpr int kScanBlock = 1024;
-constexpr int kScanBlocks = kBins / kScanBlock;        // partial sums of the bin scan
+constexpr int kScanBlocks = bins_of(kCellBits) / kScanBlock;   // partial sums of the bin scan
 static_assert(kScanBlocks >= 1 && kScanBlocks <= 2 * kScanBlock, "bin scan covers 2^10 to 2^21 bins");
+
+// Sizes from which queries are binned. Binning costs about 20 us and two scattered passes; it pays
+// once many rays share a bin. Closest hit, binned / input order, us: 250k rays 496 / 545 on 1.3M
+// random triangles but 112 / 97, 170 / 131 and 85 / 64 on a room, spheres and the Cornell box; 1M
+// rays 1398 / 1583, 282 / 301, 385 / 383, 199 / 192; 4M rays 4971 / 5790, 941 / 1123, 1200 / 1303,
+// 626 / 709. Occlusion queries end early and write one byte per ray, which binning scatters: 4M
+// rays 4254 / 4460, 472 / 485, 1033 / 1048, 427 / 373; 16M rays 16.3 / 17.3, 1.89 / 1.87,
+// 3.96 / 3.86, 1.69 / 1.44 ms.
+constexpr long long kSortClosest = 1 << 19;
+constexpr long long kSortAny = 1 << 23;
+// 64^3 cells from here on, 32^3 below: 4M rays 4.94 / 4.97 ms on the random triangles, but 1.00 / 0.94,
+// 1.29 / 1.20 and 0.70 / 0.63 ms on the others; on 2^24 rays against 10.5M triangles 32^3 cells
+// are 1.3 % slower.
+constexpr long long kFineRays = 1 << 23;
 
 __device__ __forceinline__ uint32_t spread3(uint32_t x)   // up to 7 bits -> every third bit
 {
-    x &= (uint32_t)(kCells - 1);
+    x &= 127u;
     x = (x | (x << 16)) & 0x030000FFu;
     x = (x | (x << 8)) & 0x0300F00Fu;
     x = (x | (x << 4)) & 0x030C30C3u;
@@ -38,10 +51,9 @@ __device__ __forceinline__ uint32_t spread3(uint32_t x)   // up to 7 bits -> eve
     return x;
 }
 
-__device__ __forceinline__ uint32_t cell(float v, float lo, float inv)
+__device__ __forceinline__ uint32_t cell(float v, float lo, float inv, float top)
 {
     float q = (v - lo) * inv;
-    const float top = (float)(kCells - 1);
     q = q < 0.f ? 0.f : (q > top ? top : q);
     return (uint32_t)q;
 }
@@ -79,13 +91,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
 }
 }
 
-__global__ void ray_keys_kernel(const float4* rays, long long n, float3 lo, float3 inv, uint32_t* keys, uint32_t* hist)
+__global__ void ray_keys_kernel(const float4* rays, long long n, float3 lo, float3 inv, float top, uint32_t* keys,
+                                uint32_t* hist)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     {
         float4 o = rays[2 * i], d = rays[2 * i + 1];
-        uint32_t m = (spread3(cell(o.x, lo.x, inv.x)) << 2) | (spread3(cell(o.y, lo.y, inv.y)) << 1) |
-                     spread3(cell(o.z, lo.z, inv.z));
+        uint32_t m = (spread3(cell(o.x, lo.x, inv.x, top)) << 2) | (spread3(cell(o.y, lo.y, inv.y, top)) << 1) |
+                     spread3(cell(o.z, lo.z, inv.z, top));
         uint32_t oct = (d.x < 0.f ? 4u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 1u : 0u);
         uint32_t k = (m << 3) | oct;
         keys[i] = k;
@@ -93,43 +106,43 @@ __global__ void ray_keys_kernel(const float4* rays, long long n, float3 lo, floa
     }
 }
 
-// Exclusive scan of the kBins counters in three launches: each block of 1024 scans its slice
-// and records the slice total (hist[kBins + block]); one block scans the totals (at most two
-// per thread); each block then adds its slice's offset.
-__global__ void __launch_bounds__(kScanBlock) bins_scan_kernel(uint32_t* hist)
+// Exclusive scan of the bins' counters: each block of 1024 scans its slice and records the slice
+// total (hist[bins + block]); the last block to end scans the totals (at most two per thread), which
+// the scatter adds to its slice's offsets. hist[bins + kScanBlocks] counts the blocks (zeroed with
+// the bins).
+__global__ void __launch_bounds__(kScanBlock) bins_scan_kernel(uint32_t* hist, int bins)
 {
     __shared__ uint32_t total;
+    __shared__ bool last;
     const int i = blockIdx.x * kScanBlock + threadIdx.x;
     const uint32_t v = hist[i];
     const uint32_t ex = block_exclusive_scan(v, &total);
     hist[i] = ex;
     __syncthreads();
-    if (threadIdx.x == 0) hist[kBins + blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScanBlock) bins_scan_totals_kernel(uint32_t* hist)
-{
-    __shared__ uint32_t total;
-    uint32_t* sums = hist + kBins;
-    const int t = threadIdx.x;
-    const uint32_t a = 2 * t < kScanBlocks ? sums[2 * t] : 0u;
-    const uint32_t b = 2 * t + 1 < kScanBlocks ? sums[2 * t + 1] : 0u;
-    const uint32_t ex = block_exclusive_scan(a + b, &total);
+    uint32_t* sums = hist + bins;
+    if (threadIdx.x == 0)
+    {
+        sums[blockIdx.x] = total;
+        __threadfence();
+        last = atomicAdd(&sums[kScanBlocks], 1u) == gridDim.x - 1;
+    }
     __syncthreads();
-    if (2 * t < kScanBlocks) sums[2 * t] = ex;
-    if (2 * t + 1 < kScanBlocks) sums[2 * t + 1] = ex + a;
+    if (!last) return;
+    __threadfence();
+    const int t = threadIdx.x, blocks = bins / kScanBlock;
+    const uint32_t a = 2 * t < blocks ? __ldcg(&sums[2 * t]) : 0u;
+    const uint32_t b = 2 * t + 1 < blocks ? __ldcg(&sums[2 * t + 1]) : 0u;
+    const uint32_t ex2 = block_exclusive_scan(a + b, &total);
+    if (2 * t < blocks) sums[2 * t] = ex2;
+    if (2 * t + 1 < blocks) sums[2 * t + 1] = ex2 + a;
 }
 
-__global__ void __launch_bounds__(kScanBlock) bins_scan_add_kernel(uint32_t* hist)
-{
-    hist[blockIdx.x * kScanBlock + threadIdx.x] += hist[kBins + blockIdx.x];
-}
-
-__global__ void ray_scatter_kernel(const uint32_t* keys, long long n, uint32_t* cursor, int* perm)
+__global__ void ray_scatter_kernel(const uint32_t* keys, long long n, uint32_t* cursor, int bins, int* perm)
 {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     {
-        uint32_t pos = atomicAdd(&cursor[keys[i]], 1u);
+        const uint32_t k = keys[i];
+        const uint32_t pos = cursor[bins + k / kScanBlock] + atomicAdd(&cursor[k], 1u);
         perm[pos] = (int)i;
     }
 }
@@ -195,26 +208,25 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(DevScene S, const
     }
 }
 
-// Wide-tree form: each lane traces its ray to completion; warps take rays 32 at a time from a
-// global counter (in `perm` order), so a warp that finished early takes more work. (Refilling
-// single lanes as their rays end, with the traversal state kept in registers, measured 35 %
-// slower: the binned rays of a warp stop sharing nodes and the refill logic spills.)
+// Wide-tree form: each lane traces its ray to completion; warps take `chunk` rays at a time (in
+// `perm` order), the first by their place in the grid and further ones from a global counter, so a
+// warp that finished early takes more work. The last block to end clears the counter for the next
+// launch. (Refilling single lanes as their rays end, with the traversal state kept in registers,
+// measured 35 % slower: the binned rays of a warp stop sharing nodes and the refill logic spills.)
 template <bool kAny>
 __global__ void __launch_bounds__(128) trace_fetch_wide_kernel(DevScene S, const float4* rays, const int* perm,
                                                                long long n, int4* hits, uint8_t* occluded, int lights,
-                                                               unsigned long long* next, uint32_t* status)
+                                                               unsigned long long* next, uint32_t* status, int chunk)
 {
     const int lane = threadIdx.x & 31;
-    while (true)
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk;
+    while (base < n)
     {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(next, 32ull);
-        base = __shfl_sync(kFullMask, base, 0);
-        if (base >= (unsigned long long)n) break;
-        const unsigned long long my = base + lane;
-        if (my < (unsigned long long)n)
+        const long long my = base + lane;
+        if (lane < chunk && my < n)
         {
-            const long long rid = perm ? (long long)perm[my] : (long long)my;
+            const long long rid = perm ? (long long)perm[my] : my;
             const float4 o4 = rays[2 * rid], d4 = rays[2 * rid + 1];
             const v3 o(o4.x, o4.y, o4.z), d(d4.x, d4.y, d4.z);
             Hit h;
@@ -232,7 +244,66 @@ __global__ void __launch_bounds__(128) trace_fetch_wide_kernel(DevScene S, const
             }
             if (err) atomicOr(status, err);
         }
+        if (n <= warps * chunk) return;   // every warp had one chunk: the counter is not used
+        unsigned long long got = 0;
+        if (lane == 0) got = atomicAdd(next, (unsigned long long)chunk);
+        base = warps * chunk + (long long)__shfl_sync(kFullMask, got, 0);
     }
+    if (n <= warps * chunk) return;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        // next[1]: blocks that have taken their last chunk; all have when the count is full
+        __threadfence();
+        if (atomicAdd(next + 1, 1ull) == gridDim.x - 1)
+        {
+            next[0] = 0;
+            next[1] = 0;
+        }
+    }
+}
+
+namespace
+{
+// Rays a warp takes at a time: 32, or fewer (a power of two) while the query still has no more
+// chunks than the GPU holds warps (4256 at 72 registers). A small query is a chain of dependent
+// node visits, and a warp visits the union of its rays' branches: 1000 rays 37 -> 21 us in a room
+// of 48k triangles, 173 -> 112 us against 1.3M random triangles, 16,000 rays 43 -> 36 and
+// 197 -> 136 us. Twice or four times the warps a GPU holds lose that again (16,000 rays 145 and
+// 160 us), at 130,000 rays and above 32 a warp are best.
+int chunk_for(long long n, long long warps)
+{
+    int chunk = 1;
+    while (chunk < 32 && chunk * warps < n) chunk *= 2;
+    return chunk;
+}
+
+template <bool kAny>
+void launch_wide(const DevScene& S, const float4* rays, const int* order, long long n, void* out, int lights, int sms,
+                 unsigned long long* next, uint32_t* status, cudaStream_t st)
+{
+    const int perSm = occupancy_blocks_per_sm((const void*)trace_fetch_wide_kernel<kAny>, 128);
+    const long long full = (long long)sms * perSm;
+    const int chunk = chunk_for(n, 4 * full);
+    const long long need = (n + 4ll * chunk - 1) / (4ll * chunk);
+    trace_fetch_wide_kernel<kAny><<<(int)std::min(full, need), 128, 0, st>>>(
+        S, rays, order, n, kAny ? nullptr : (int4*)out, kAny ? (uint8_t*)out : nullptr, lights, next, status, chunk);
+}
+
+void sort_rays(const float4* rays, long long n, const float lo[3], const float hi[3], int sms, uint32_t* keys,
+               uint32_t* hist, int* perm, cudaStream_t st)
+{
+    const int cellBits = n >= kFineRays ? kCellBits : kCellBits - 1;
+    const int bins = bins_of(cellBits), cells = 1 << cellBits;
+    const float3 flo = make_float3(lo[0], lo[1], lo[2]);
+    auto inv = [&](float a, float b) { return b > a ? (float)cells / (b - a) : 0.0f; };
+    const float3 finv = make_float3(inv(lo[0], hi[0]), inv(lo[1], hi[1]), inv(lo[2], hi[2]));
+    cudaMemsetAsync(hist, 0, sizeof(uint32_t) * ((size_t)bins + kScanBlocks + 1), st);   // bins and block count
+    const int g = (int)std::min<long long>(sms * 8, (n + 255) / 256);
+    ray_keys_kernel<<<g, 256, 0, st>>>(rays, n, flo, finv, (float)(cells - 1), keys, hist);
+    bins_scan_kernel<<<bins / kScanBlock, kScanBlock, 0, st>>>(hist, bins);
+    ray_scatter_kernel<<<g, 256, 0, st>>>(keys, n, hist, bins, perm);
+}
 }
 
 int launch_trace_binned(const DevScene& S, const float4* rays, long long n, void* out, bool any, int lights,
@@ -246,39 +317,20 @@ int launch_trace_binned(const DevScene& S, const float4* rays, long long n, void
     const int* order = nullptr;
     if (binning)
     {
-        float3 flo = make_float3(lo[0], lo[1], lo[2]);
-        auto inv = [](float a, float b) { return b > a ? (float)kCells / (b - a) : 0.0f; };
-        float3 finv = make_float3(inv(lo[0], hi[0]), inv(lo[1], hi[1]), inv(lo[2], hi[2]));
-        cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kBins, st);
-        int g = sms * 8;
-        ray_keys_kernel<<<g, 256, 0, st>>>(rays, n, flo, finv, keys, hist);
-        bins_scan_kernel<<<kScanBlocks, kScanBlock, 0, st>>>(hist);
-        bins_scan_totals_kernel<<<1, kScanBlock, 0, st>>>(hist);
-        bins_scan_add_kernel<<<kScanBlocks, kScanBlock, 0, st>>>(hist);
-        ray_scatter_kernel<<<g, 256, 0, st>>>(keys, n, hist, perm);
+        sort_rays(rays, n, lo, hi, sms, keys, hist, perm, st);
         order = perm;
     }
-    cudaMemsetAsync(next, 0, sizeof(unsigned long long), st);
-    int per_sm = 0;
     if (S.wnodes && S.wideOn)
     {
+        if (evStart) cudaEventRecord(evStart, st);
         if (any)
-        {
-            per_sm = occupancy_blocks_per_sm((const void*)trace_fetch_wide_kernel<true>, 128);
-            if (evStart) cudaEventRecord(evStart, st);
-            trace_fetch_wide_kernel<true><<<sms * (per_sm > 0 ? per_sm : 1), 128, 0, st>>>(
-                S, rays, order, n, nullptr, (uint8_t*)out, lights, next, status);
-        }
+            launch_wide<true>(S, rays, order, n, out, lights, sms, next, status, st);
         else
-        {
-            per_sm = occupancy_blocks_per_sm((const void*)trace_fetch_wide_kernel<false>, 128);
-            if (evStart) cudaEventRecord(evStart, st);
-            trace_fetch_wide_kernel<false><<<sms * (per_sm > 0 ? per_sm : 1), 128, 0, st>>>(
-                S, rays, order, n, (int4*)out, nullptr, lights, next, status);
-        }
+            launch_wide<false>(S, rays, order, n, out, lights, sms, next, status, st);
         if (evStop) cudaEventRecord(evStop, st);
         return (int)cudaGetLastError();
     }
+    int per_sm = 0;
     if (evStart) cudaEventRecord(evStart, st);
     if (any)
     {
@@ -293,8 +345,11 @@ int launch_trace_binned(const DevScene& S, const float4* rays, long long n, void
             S, rays, order, n, (int4*)out, nullptr, lights, next, status);
     }
     if (evStop) cudaEventRecord(evStop, st);
+    cudaMemsetAsync(next, 0, sizeof(unsigned long long), st);   // the counter is zero between launches
     return (int)cudaGetLastError();
 }
 
-int trace_bins() { return kBins + kScanBlocks; }   // counters + scan partial sums
+bool trace_sorts(long long n, bool any) { return n >= (any ? kSortAny : kSortClosest); }
+
+int trace_bins() { return bins_of(kCellBits) + kScanBlocks + 1; }   // counters, scan partial sums, block count
 }
