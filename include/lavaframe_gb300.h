@@ -357,8 +357,8 @@ lf_status lf_write_jpg(const char* path, const uint8_t* rgb8, int32_t width, int
  * samples [first_sample, first_sample + count) of `p` into the caller's device buffer
  * `d_accum` (width*height float4 RGBA32F, row 0 = bottom, A unused; zero it before the first
  * call), in sample order; the sums are bit-identical to lf_frame_render's.
- * All wavefront state lives in one fixed device array of the library (30 MiB + 256 B, i.e.
- * 31.5 MB, on every GPU that loads it, held until exit): one tile (tile_width x tile_height,
+ * All wavefront state lives in one fixed device array of the library (32.5 MiB + 1 KiB, i.e.
+ * 34.1 MB, on every GPU that loads it, held until exit): one tile (tile_width x tile_height,
  * or the whole frame) may have at most 131072 pixels, larger tiles are rejected with
  * LF_ERR_INVALID. The call makes no cudaMalloc/cudaFree and no allocating library call.
  * The first call on a device resolves the array's address (cudaGetSymbolAddress); make it

@@ -2,6 +2,8 @@
 // The per-path work is the same code as the per-batch frame kernels (lf_pathops.cuh); only
 // the bookkeeping differs: paths find their job through info.w, finished paths hand their
 // slot to a new path, and pass completion is counted on the device.
+#include <algorithm>
+
 #include "lf_engine.h"
 #include "lf_pathops.cuh"
 
@@ -113,7 +115,78 @@ __device__ __forceinline__ unsigned long long find_pass(const EnginePass* passes
 }
 }
 
-// ------------------------------------------------------------------ init / append / reset
+namespace
+{
+
+// Clears the work counters of a step.
+__device__ __forceinline__ void reset_step(EngineCtl* c)
+{
+    c->shadowCount = 0;
+    c->extendNext = 0;
+    c->shadeNext = 0;
+    c->shadowNext = 0;
+    c->hitCount = 0;
+    c->missCount = 0;
+    for (int k = 0; k < 4; ++k) c->bucketCount[k] = 0;
+}
+
+// Whether this is the last block of the grid to get here (every thread of it has done its work);
+// the counter is left at zero. Called by every block, by all its threads.
+__device__ __forceinline__ bool last_block(int* counter)
+{
+    __syncthreads();
+    bool last = false;
+    if (threadIdx.x == 0)
+    {
+        __threadfence();
+        last = atomicAdd(counter, 1) == (int)gridDim.x - 1;
+        if (last) *counter = 0;
+    }
+    return last;   // of thread 0; false elsewhere
+}
+
+// A kernel's share of n queue entries: warps take `chunk` entries at a time, the first chunk by
+// their place in the grid and further ones from a counter, so that long rays do not hold up a
+// fixed share and a queue of one chunk per warp needs no atomics (8,500 of them on one address
+// cost about 8 us). The chunk is 32, or fewer (a power of two) while the entries do not give every
+// warp of the grid a chunk: a thin queue is a chain of dependent loads per path, and a warp runs
+// the union of its lanes' branches (20,000 paths on spheres 1189 -> 755 us, in a room 667 -> 486).
+struct QueueShare
+{
+    int n, chunk, base;
+
+    __device__ __forceinline__ explicit QueueShare(int entries) : n(entries), chunk(32)
+    {
+        const int warps = gridDim.x * (blockDim.x >> 5);
+        while (chunk > 1 && (long long)(chunk >> 1) * warps >= n) chunk >>= 1;
+        const long long first = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk;
+        base = first < n ? (int)first : n;
+    }
+    __device__ __forceinline__ bool more() const { return base < n; }
+    // this lane's entry, or -1
+    __device__ __forceinline__ int entry() const
+    {
+        const int lane = threadIdx.x & 31;
+        return lane < chunk && base + lane < n ? base + lane : -1;
+    }
+    // the warp's next chunk; every lane calls
+    __device__ __forceinline__ void next(int* counter)
+    {
+        const long long once = (long long)gridDim.x * (blockDim.x >> 5) * chunk;
+        if (n <= once)
+        {
+            base = n;
+            return;
+        }
+        int got = 0;
+        if ((threadIdx.x & 31) == 0) got = atomicAdd(counter, chunk);
+        got = __shfl_sync(kFull, got, 0);
+        base = got < n - (int)once ? (int)once + got : n;
+    }
+};
+}
+
+// ------------------------------------------------------------------ init / append
 __global__ void engine_init_kernel(EngineBuffers b)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < b.cap; i += gridDim.x * blockDim.x)
@@ -130,6 +203,9 @@ __global__ void engine_init_kernel(EngineBuffers b)
         b.ctl->count[0] = 0;
         b.ctl->count[1] = 0;
         b.ctl->shadowCount = 0;
+        b.ctl->refillDone = 0;
+        b.ctl->shadowDone = 0;
+        reset_step(b.ctl);
     }
 }
 
@@ -147,26 +223,6 @@ __global__ void engine_append_kernel(EngineBuffers b, unsigned long long total, 
         ++lo;
     }
     c->passLo = lo;
-}
-
-// After finish and refill: count the refilled slots as taken and their ids as issued, and
-// clear the lists and counters the rest of the step fills.
-__global__ void engine_reset_kernel(EngineCtl* c, int parity)
-{
-    c->freeCount -= c->taken;
-    c->next += (unsigned long long)c->taken;
-    c->active += c->taken;
-    c->taken = 0;
-    c->doneCount[parity] = 0;
-    c->shadowCount = 0;
-    c->count[parity ^ 1] = 0;
-    c->extendNext = 0;
-    c->shadeNext = 0;
-    c->shadowNext = 0;
-    c->refillNext = 0;
-    c->hitCount = 0;
-    c->missCount = 0;
-    for (int k = 0; k < 4; ++k) c->bucketCount[k] = 0;
 }
 
 // ------------------------------------------------------------------ finish / refill
@@ -251,8 +307,11 @@ __global__ void __launch_bounds__(kRefillBlock) engine_refill_kernel(EngineBuffe
     const int freeCount = ctl->freeCount;
     const unsigned long long left = next < total ? total - next : 0ull;
     const int m = (int)((unsigned long long)freeCount < left ? (unsigned long long)freeCount : left);
-    if (m <= 0) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->taken = m;
+    if (m <= 0)
+    {
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->doneCount[parity] = 0;
+        return;
+    }
     const unsigned long long plo = ctl->passLo, phi = ctl->numPasses;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -381,6 +440,15 @@ __global__ void __launch_bounds__(kRefillBlock) engine_refill_kernel(EngineBuffe
             }
         }
     }
+    if (last_block(&ctl->refillDone))
+    {
+        // the step's new paths are started: commit them
+        ctl->freeCount -= m;
+        ctl->next += (unsigned long long)m;
+        ctl->active += m;
+        ctl->refillNext = 0;
+        ctl->doneCount[parity] = 0;
+    }
 }
 
 // ------------------------------------------------------------------ extend / shade / shadow
@@ -393,18 +461,13 @@ __global__ void __maxnreg__(72) engine_extend_kernel(EngineBuffers b, EngineJob 
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&b.ctr[1], (unsigned long long)n);
     const int* q = b.queue[parity];
     const int lane = threadIdx.x & 31;
-    while (true)
+    for (QueueShare share(n); share.more(); share.next(&b.ctl->extendNext))
     {
-        // warps take queue entries 32 at a time, so long rays do not hold up a fixed share
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&b.ctl->extendNext, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const int i = base + lane;
+        const int i = share.entry();
         int p = -1;
         bool miss = false;
         int cls = 0;
-        if (i < n)
+        if (i >= 0)
         {
             p = q[i];
             const float4 o4 = b.ps.o[p], d4 = b.ps.d[p];
@@ -486,19 +549,15 @@ __global__ void __launch_bounds__(256, kThreadsPerSm ? kThreadsPerSm / 256 : 1)
     const int nHit = ctl->hitCount;   // part: hits at [0, nHit), misses at the back
     int* qout = b.queue[parity ^ 1];
     const int lane = threadIdx.x & 31;
-    while (true)
+    for (QueueShare share(n); share.more(); share.next(&ctl->shadeNext))
     {
-        // warps take 32 queue entries at a time and append their outputs with one atomic per
-        // queue, so no warp waits for the others of its block
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&ctl->shadeNext, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const int i = base + lane;
+        // warps append their outputs with one atomic per queue, so no warp waits for the others of
+        // its block
+        const int i = share.entry();
         bool pushExt = false, pushShadow = false;
         int p = -1;
         ShadowRec rec;
-        if (i < n)
+        if (i >= 0)
         {
             if (i >= nHit)
                 p = b.part[b.cap - 1 - (i - nHit)];
@@ -558,22 +617,17 @@ __global__ void __launch_bounds__(256, kThreadsPerSm ? kThreadsPerSm / 256 : 1)
 }
 
 template <bool kOne>
-__global__ void __maxnreg__(72) engine_shadow_kernel(EngineBuffers b, EngineJob one)
+__global__ void __maxnreg__(72) engine_shadow_kernel(EngineBuffers b, EngineJob one, int parity)
 {
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
     const int n = b.ctl->shadowCount;
     unsigned long long rays = 0;
-    const int lane = threadIdx.x & 31;
-    while (true)
+    for (QueueShare share(n); share.more(); share.next(&b.ctl->shadowNext))
     {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&b.ctl->shadowNext, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const int i = base + lane;
-        if (i >= n) continue;
+        const int i = share.entry();
+        if (i < 0) continue;
         const ShadowRec* rec = b.shadow + i;
         float4 L;
         if constexpr (kOne)
@@ -593,6 +647,11 @@ __global__ void __maxnreg__(72) engine_shadow_kernel(EngineBuffers b, EngineJob 
     }
     warp_count_add(&b.ctr[2], rays);
     block_done_end(b, td, bd);
+    if (last_block(&b.ctl->shadowDone))
+    {
+        b.ctl->count[parity] = 0;   // the next step's shade fills this queue
+        reset_step(b.ctl);
+    }
 }
 
 // ------------------------------------------------------------------ drain
@@ -603,56 +662,135 @@ __global__ void __maxnreg__(72) engine_shadow_kernel(EngineBuffers b, EngineJob 
 // sequence per bounce whose length is set by the slowest ray of an almost empty pool.
 // One path from its queued extension ray to its end; returns the extension and shadow rays
 // it traced.
-__device__ __forceinline__ void drain_path(const EngineBuffers& b, const EngineJob& J, int p, unsigned long long& ext,
-                                           unsigned long long& shadowRays)
+template <bool kLights = true>
+__device__ __forceinline__ void run_path(const ShadeScene& S, const Params& P, const PathSoA& ps, uint32_t* status,
+                                         unsigned long long* ctr, int p, unsigned long long& ext,
+                                         unsigned long long& shadowRays)
 {
     for (int bounce = 0; bounce < 4096; ++bounce)
     {
-        const float4 o4 = b.ps.o[p], d4 = b.ps.d[p];
+        const float4 o4 = ps.o[p], d4 = ps.d[p];
         Hit h;
-        const uint32_t err = closest_hit<false>(J.S.trav, f3(o4), f3(d4), kInfinity, J.P.useLights != 0, &h, nullptr);
-        b.ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));
-        set_error(b.status, err);
+        const uint32_t err = closest_hit<false>(S.trav, f3(o4), f3(d4), kInfinity, P.useLights != 0, &h, nullptr);
+        ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));
+        set_error(status, err);
         ++ext;
         bool pushExt = false, pushShadow = false;
         ShadowRec rec;
-        shade_path(J.S, J.P, b.ps, p, b.ctr, pushExt, pushShadow, rec);
-        if (pushShadow) set_error(b.status, shadow_path(J.S, J.P, b.ps, &rec, shadowRays));
+        shade_path<kLights>(S, P, ps, p, ctr, pushExt, pushShadow, rec);
+        if (pushShadow) set_error(status, shadow_path(S, P, ps, &rec, shadowRays));
         if (!pushExt) return;
     }
 }
 
+// More than `limit` queued paths are left for the step kernels.
 template <bool kOne>
-__global__ void __launch_bounds__(128) engine_drain_kernel(EngineBuffers b, EngineJob one, int parity)
+__global__ void __launch_bounds__(128) engine_drain_kernel(EngineBuffers b, EngineJob one, int parity, int limit)
 {
+    if (b.ctl->count[parity] > limit || b.ctl->count[parity] == 0) return;
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
     EngineCtl* ctl = b.ctl;
     const int n = ctl->count[parity];
     const int* q = b.queue[parity];
-    const int lane = threadIdx.x & 31;
     unsigned long long ext = 0, shadowRays = 0;
-    while (true)
+    for (QueueShare share(n); share.more(); share.next(&ctl->extendNext))
     {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&ctl->extendNext, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const int i = base + lane;
-        if (i < n)
+        const int i = share.entry();
+        if (i >= 0)
         {
             const int p = q[i];
             if constexpr (kOne)
-                drain_path(b, one, p, ext, shadowRays);
+                run_path(one.S, one.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
             else
-                drain_path(b, b.jobs[job_of(reinterpret_cast<const int*>(b.ps.info)[4 * p + 3])], p, ext, shadowRays);
+            {
+                const EngineJob& J = b.jobs[job_of(reinterpret_cast<const int*>(b.ps.info)[4 * p + 3])];
+                run_path(J.S, J.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
+            }
             end_path(b, p, b.ps.info[p], b.ps.L[p], td, bd);
         }
     }
     warp_count_add(&b.ctr[1], ext);
     warp_count_add(&b.ctr[2], shadowRays);
     block_done_end(b, td, bd);
+    if (last_block(&ctl->shadowDone))
+    {
+        ctl->count[parity] = 0;
+        reset_step(ctl);
+    }
+}
+
+// ------------------------------------------------------------------ runs on the idle pool
+// Starts path i of a run in slot `slot(Q, entry)` (entry: its place in the radiance of its pass
+// Q); returns the slot. Pass k of the table is the last one with pathBase <= i.
+template <class Slot>
+__device__ __forceinline__ int start_path(const PathSoA& ps, const Params& P, const EnginePass& first,
+                                          const EnginePass* table, int numPasses, int i, bool keepPass, Slot slot)
+{
+    int k = 0;
+    for (int hi = numPasses; hi - k > 1;)
+    {
+        const int mid = (k + hi) >> 1;
+        if (table[mid].pathBase <= (unsigned long long)i) k = mid;
+        else hi = mid;
+    }
+    EnginePass Q = first;
+    if (numPasses > 1) Q = table[k];
+    const int local = i - (int)Q.pathBase;
+    const int visPix = Q.visW * Q.visH;
+    const int s = local / visPix;
+    int lx, ly;
+    pixel_of(local - s * visPix, Q.visW, Q.visH, lx, ly);
+    const int entry = s * visPix + ly * Q.visW + lx;
+    const int p = slot(Q, entry);
+    ps.L[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+    ps.info[p] = make_int4(entry, 0, 0, keepPass ? k : -1);
+    gen_path(P, Q.tileX, Q.tileY, Q.tileOrdinal, Q.firstSample + s, lx, ly, ps, p);
+    return p;
+}
+
+// Every path of a run, path i in slot i, queued in order, so that the pool need not be searched for
+// free slots.
+__global__ void __launch_bounds__(256) engine_start_kernel(EngineBuffers b, Params P, EnginePass first, EnginePass* table,
+                                                           int numPasses, int n)
+{
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid == 0)
+    {
+        if (numPasses == 1) table[0] = first;
+        b.ctl->count[0] = n;
+        b.ctl->freeCount -= n;
+        b.ctl->active += n;
+    }
+    for (int i = tid; i < n; i += gridDim.x * blockDim.x)
+        b.queue[0][i] = start_path(b.ps, P, first, table, numPasses, i, true, [&](const EnginePass&, int) { return i; });
+}
+
+// A whole small run in one launch: every thread takes paths from their camera ray to their end
+// (the operations of the step kernels in their order, so results and ray counts are unchanged),
+// without queues. b.ps.L is the run's radiance array: a path's slot is its radiance entry, so an
+// ended path needs no write-out, and the slots stay marked free (info.w = -1). kDirectPaths
+// says where it pays.
+template <bool kLights>
+__global__ void __launch_bounds__(128) engine_direct_kernel(EngineBuffers b, EngineJob one, EnginePass first,
+                                                            const EnginePass* table, int numPasses, int n)
+{
+    unsigned long long ext = 0, shadowRays = 0;
+    for (QueueShare share(n); share.more(); share.next(&b.ctl->extendNext))
+    {
+        const int i = share.entry();
+        if (i >= 0)
+        {
+            const int p = start_path(b.ps, one.P, first, table, numPasses, i, false,
+                                     [](const EnginePass& Q, int entry) { return (int)Q.pathBase + entry; });
+            if (one.P.maxDepth > 0) run_path<kLights>(one.S, one.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
+        }
+        __syncwarp();
+    }
+    warp_count_add(&b.ctr[1], ext);
+    warp_count_add(&b.ctr[2], shadowRays);
+    if (last_block(&b.ctl->shadowDone)) b.ctl->extendNext = 0;
 }
 
 // ------------------------------------------------------------------ accumulate
@@ -694,9 +832,68 @@ __global__ void engine_accumulate_kernel(int width, int tileW, int tileH, Engine
     }
 }
 
+// The same for every pixel of a frame over a run's passes: chunk c of the tile in row ty, column tx
+// is pass c * tiles + (tilesY - 1 - ty) * tilesX + tx.
+__global__ void engine_accumulate_run_kernel(int width, int height, int tileW, int tileH, const EnginePass* table,
+                                             int chunks, int tilesX, int tilesY, float4* accum, double* accum64)
+{
+    for (int gpix = blockIdx.x * blockDim.x + threadIdx.x; gpix < width * height; gpix += gridDim.x * blockDim.x)
+    {
+        const int x = gpix % width, y = gpix / width;
+        const int tx = x / tileW, ty = y / tileH;
+        const int tile = (tilesY - 1 - ty) * tilesX + tx;
+        float4 a = accum[gpix];
+        double ax = 0, ay = 0, az = 0;
+        if (accum64)
+        {
+            ax = accum64[gpix * 3 + 0];
+            ay = accum64[gpix * 3 + 1];
+            az = accum64[gpix * 3 + 2];
+        }
+        for (int c = 0; c < chunks; ++c)
+        {
+            const EnginePass& Q = table[c * tilesX * tilesY + tile];
+            const int visPix = Q.visW * Q.visH, lp = (y - ty * tileH) * Q.visW + (x - tx * tileW);
+            for (int s = 0; s < Q.nSamples; ++s)
+            {
+                const float4 l = Q.radiance[(size_t)s * visPix + lp];
+                a.x = a.x + l.x;
+                a.y = a.y + l.y;
+                a.z = a.z + l.z;
+                if (accum64)
+                {
+                    ax += (double)l.x;
+                    ay += (double)l.y;
+                    az += (double)l.z;
+                }
+            }
+        }
+        accum[gpix] = a;
+        if (accum64)
+        {
+            accum64[gpix * 3 + 0] = ax;
+            accum64[gpix * 3 + 1] = ay;
+            accum64[gpix * 3 + 2] = az;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ launchers
 namespace
 {
+// Runs of up to kDirectPaths paths are traced by one launch. Kernel by kernel every bounce waits for
+// its slowest ray three times over; one thread per path overlaps those waits, but its code (traversal,
+// shading and occlusion in one kernel) overflows the instruction caches once the GPU is full (15 of
+// 24 stall cycles per issue at 262k paths). One launch / kernel by kernel, us: 4096 paths 113 / 166
+// (Cornell box), 266 / 386 (room), 214 / 400 (random triangles), 200 / 412 (spheres); 62k paths
+// 204 / 231, 549 / 587, 594 / 678, 477 / 771; 131k paths 388 / 254, 957 / 732, 776 / 917, 657 / 996.
+constexpr int kDirectPaths = 1 << 16;
+// A run takes its paths to their ends in the drain after the second or fourth bounce once this many
+// are left: spheres 262k paths 1321 -> 1104 us, room 1M paths 2073 -> 2092; with 65,536 the room's
+// 2148, with 16,384 the spheres' 524k paths 1272 -> 1360.
+constexpr int kDrainPaths = 1 << 15;
+constexpr int kRunBounces = 16;   // bounces of a run in steps; deeper paths are taken to their ends by the drain
+
 int sm_count()
 {
     static int n = 0;
@@ -736,55 +933,99 @@ int launch_engine_append(const EngineBuffers& b, unsigned long long total, unsig
 namespace
 {
 template <bool kOne>
-void step(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream_t st)
+void refill(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream_t st)
 {
     const int BF = 256;
-    engine_finish_kernel<<<full_grid((const void*)engine_finish_kernel, BF, b.cap), BF, 0, st>>>(b, parity);
+    if (!kOne || one.P.maxDepth <= 0)   // only depth-0 paths are on the done list
+        engine_finish_kernel<<<full_grid((const void*)engine_finish_kernel, BF, b.cap), BF, 0, st>>>(b, parity);
     engine_refill_kernel<kOne><<<full_grid((const void*)engine_refill_kernel<kOne>, kRefillBlock,
                                            (long long)b.cap / kRefillGroups),
                                  kRefillBlock, 0, st>>>(b, one, parity);
-    engine_reset_kernel<<<1, 1, 0, st>>>(b.ctl, parity);
+}
+
+// One bounce of the queued paths, at most n of them.
+template <bool kOne>
+void bounce(const EngineBuffers& b, const EngineJob& one, int parity, int n, cudaStream_t st)
+{
     const int be = b.blockExtend > 0 ? b.blockExtend : 128;
     const int bs = b.blockShade > 0 ? b.blockShade : 128;
     const int bw = b.blockShadow > 0 ? b.blockShadow : 128;
-    engine_extend_kernel<kOne><<<full_grid((const void*)engine_extend_kernel<kOne>, be, b.cap), be, 0, st>>>(b, one,
-                                                                                                           parity);
-    if (b.shadeThreadsPerSm == 512 && kOne && !one.P.useLights)
-        engine_shade_kernel<kOne, 512, false><<<full_grid((const void*)engine_shade_kernel<kOne, 512, false>, bs, b.cap),
-                                                bs, 0, st>>>(b, one, parity);
-    else if (b.shadeThreadsPerSm == 512)
-        engine_shade_kernel<kOne, 512><<<full_grid((const void*)engine_shade_kernel<kOne, 512>, bs, b.cap), bs, 0, st>>>(
-            b, one, parity);
+    // grids for one path per warp at least: thin queues are spread over the GPU (QueueShare)
+    auto grid = [&](const void* k, int block) { return full_grid(k, block, (long long)n * 32); };
+    auto shade = [&](auto kernel) { kernel<<<grid((const void*)kernel, bs), bs, 0, st>>>(b, one, parity); };
+    engine_extend_kernel<kOne><<<grid((const void*)engine_extend_kernel<kOne>, be), be, 0, st>>>(b, one, parity);
+    const bool lights = !kOne || one.P.useLights;
+    if (b.shadeThreadsPerSm == 512)
+        lights ? shade(engine_shade_kernel<kOne, 512>) : shade(engine_shade_kernel<kOne, 512, false>);
     else if (b.shadeThreadsPerSm == 768)
-        engine_shade_kernel<kOne, 768><<<full_grid((const void*)engine_shade_kernel<kOne, 768>, bs, b.cap), bs, 0, st>>>(
-            b, one, parity);
-    else if (b.shadeThreadsPerSm == 1024 && kOne && !one.P.useLights)
-        engine_shade_kernel<kOne, 1024, false><<<full_grid((const void*)engine_shade_kernel<kOne, 1024, false>, bs, b.cap),
-                                                 bs, 0, st>>>(b, one, parity);
+        shade(engine_shade_kernel<kOne, 768>);
     else if (b.shadeThreadsPerSm == 1024)
-        engine_shade_kernel<kOne, 1024><<<full_grid((const void*)engine_shade_kernel<kOne, 1024>, bs, b.cap), bs, 0,
-                                          st>>>(b, one, parity);
+        lights ? shade(engine_shade_kernel<kOne, 1024>) : shade(engine_shade_kernel<kOne, 1024, false>);
     else
-        engine_shade_kernel<kOne, 0><<<full_grid((const void*)engine_shade_kernel<kOne, 0>, bs, b.cap), bs, 0, st>>>(
-            b, one, parity);
-    engine_shadow_kernel<kOne><<<full_grid((const void*)engine_shadow_kernel<kOne>, bw, b.cap), bw, 0, st>>>(b, one);
+        shade(engine_shade_kernel<kOne, 0>);
+    engine_shadow_kernel<kOne><<<grid((const void*)engine_shadow_kernel<kOne>, bw), bw, 0, st>>>(b, one, parity);
 }
+
+template <bool kOne>
+void step(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream_t st)
+{
+    refill<kOne>(b, one, parity, st);
+    bounce<kOne>(b, one, parity, b.cap, st);
+}
+
+template <bool kOne>
+void drain(const EngineBuffers& b, const EngineJob& one, int parity, int n, int limit, cudaStream_t st)
+{
+    engine_drain_kernel<kOne><<<full_grid((const void*)engine_drain_kernel<kOne>, 128, (long long)n * 32), 128, 0, st>>>(
+        b, one, parity, limit);
 }
 
 template <bool kOne>
 void drain_step(const EngineBuffers& b, const EngineJob& one, cudaStream_t st)
 {
-    const int BF = 256;
     for (int parity = 0; parity < 2; ++parity)
     {
-        engine_finish_kernel<<<full_grid((const void*)engine_finish_kernel, BF, b.cap), BF, 0, st>>>(b, parity);
-        engine_refill_kernel<kOne><<<full_grid((const void*)engine_refill_kernel<kOne>, kRefillBlock,
-                                               (long long)b.cap / kRefillGroups),
-                                     kRefillBlock, 0, st>>>(b, one, parity);
-        engine_reset_kernel<<<1, 1, 0, st>>>(b.ctl, parity);
-        engine_drain_kernel<kOne><<<full_grid((const void*)engine_drain_kernel<kOne>, 128, b.cap), 128, 0, st>>>(
-            b, one, parity);
+        refill<kOne>(b, one, parity, st);
+        drain<kOne>(b, one, parity, b.cap, b.cap, st);
     }
+}
+}
+
+int launch_frame_run(const EngineBuffers& b0, const EngineJob& one, const EnginePass& first, EnginePass* table,
+                     int numPasses, int n, float4* radiance, int drainPaths, cudaStream_t st)
+{
+    EngineBuffers b = b0;
+    b.passes = table;
+    if (one.P.maxDepth <= 0 || n <= std::min(kDirectPaths, drainPaths))
+    {
+        b.ps.L = radiance;
+        auto direct = [&](auto kernel) {
+            kernel<<<full_grid((const void*)kernel, 128, (long long)n * 32), 128, 0, st>>>(b, one, first, table, numPasses,
+                                                                                          n);
+        };
+        one.P.useLights ? direct(engine_direct_kernel<true>) : direct(engine_direct_kernel<false>);
+        return (int)cudaGetLastError();
+    }
+    engine_start_kernel<<<full_grid((const void*)engine_start_kernel, 256, n), 256, 0, st>>>(b, one.P, first, table,
+                                                                                             numPasses, n);
+    const int bounces = std::min(one.P.maxDepth, kRunBounces);
+    for (int k = 0; k < bounces; ++k)
+    {
+        if ((k == 2 || k == 4) && bounces - k > 1) drain<true>(b, one, k & 1, n, std::min(kDrainPaths, drainPaths), st);
+        bounce<true>(b, one, k & 1, n, st);
+    }
+    if (bounces < one.P.maxDepth) drain<true>(b, one, bounces & 1, n, n, st);
+    return (int)cudaGetLastError();
+}
+
+int launch_engine_accumulate_run(const Params& P, const EnginePass* table, int chunks, int tilesX, int tilesY,
+                                 float4* accum, double* accum64, cudaStream_t st)
+{
+    const int B = 256;
+    const long long pix = (long long)P.width * P.height;
+    engine_accumulate_run_kernel<<<full_grid((const void*)engine_accumulate_run_kernel, B, pix), B, 0, st>>>(
+        P.width, P.height, P.tileW, P.tileH, table, chunks, tilesX, tilesY, accum, accum64);
+    return (int)cudaGetLastError();
 }
 
 int launch_engine_drain(const EngineBuffers& b, const EngineJob* one, cudaStream_t st)

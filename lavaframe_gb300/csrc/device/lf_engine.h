@@ -10,17 +10,23 @@
 // image sums are the ones of the per-batch pipeline, bit for bit.
 //
 // One engine step with parity k (graph-captured, two steps per graph so the parity returns):
-//   finish   done[k] (paths of depth-0 jobs): write them out, count pass completions, free
-//            their slots
-//   refill   start new paths in free slots while unissued ids remain (-> queue[k])
-//   reset    commit the refill, clear done[k], the shadow queue and queue[k^1]
+//   finish   done[k] (paths of depth-0 jobs; not launched for a single job that traces): write
+//            them out, count pass completions, free their slots
+//   refill   start new paths in free slots while unissued ids remain (-> queue[k]); its last
+//            block commits the ids and clears done[k]
 //   extend   closest hit of every queued path; hits and misses -> part (front and back), or
 //            with sort-by-material the hits into one bucket per material class
 //   shade    one PathTrace bounce over part's hits, then its misses, so that a warp shades
 //            one kind; survivors -> queue[k^1]; a path that ends without next-event rays is
 //            written out (radiance into its pass, completion counted, slot freed) on the spot
-//   shadow   next-event visibility; writes out the paths that ended at the record's vertex
+//   shadow   next-event visibility; writes out the paths that ended at the record's vertex; its
+//            last block clears queue[k] and the step's counters for the next step
 //   (the drain kernel writes out each path it runs to its end)
+//
+// A frame run whose paths fit the idle pool needs none of the bookkeeping between steps: one
+// launch starts every path (start), then extend, shade and shadow run once per bounce up to the
+// job's depth, without a look at the device from the host (launch_frame_run); a small
+// run is one launch altogether.
 #pragma once
 
 #include "lf_kernels.h"
@@ -30,6 +36,7 @@ namespace lfd
 constexpr int kPassRingBits = 14;
 constexpr int kPassRing = 1 << kPassRingBits;   // pass descriptors in flight
 constexpr int kMaxEngineJobs = 1 << 16;         // job slots (packed into the upper bits of info.w)
+constexpr int kDefaultShadeCap = 512;           // shade kernel register cap (threads per SM)
 
 struct EngineJob
 {
@@ -62,6 +69,7 @@ struct EngineCtl
     int taken;                     // slots the current step's refill started
     int extendNext, shadeNext, shadowNext;   // work counters of the extend, shade and shadow kernels
     int refillNext;                // ids handed out by the current refill
+    int refillDone, shadowDone;    // blocks that have ended (the last one resets the step's counters)
     int hitCount, missCount;       // the extension queue split by extend: hits, then misses
     int bucketCount[4];            // sort-by-material: hits per material class
 };
@@ -94,6 +102,17 @@ int launch_engine_step(const EngineBuffers& b, const EngineJob* one, int parity,
 // shadow kernels are replaced by one kernel that runs every queued path to its end (one thread
 // per path) and queues it as done. Leaves the parity where a step pair leaves it.
 int launch_engine_drain(const EngineBuffers& b, const EngineJob* one, cudaStream_t st);
+// A whole run of one job on the idle pool: n <= cap paths of numPasses passes in the table
+// (= b.passes; `first` is written there when the run has one pass), whose pathBase counts from 0 in
+// increasing order and whose radiance lies at radiance + pathBase. Small runs are traced by one
+// launch, larger ones by one launch per kernel and bounce. drainPaths bounds the paths that one thread each
+// takes to their ends.
+int launch_frame_run(const EngineBuffers& b, const EngineJob& one, const EnginePass& first, EnginePass* table,
+                     int numPasses, int n, float4* radiance, int drainPaths, cudaStream_t st);
+// Per-pixel sums of a run's passes - chunks of samples, each with every tile in TiledRenderer's
+// order (top row first) - in sample order.
+int launch_engine_accumulate_run(const Params& P, const EnginePass* table, int chunks, int tilesX, int tilesY,
+                                 float4* accum, double* accum64, cudaStream_t st);
 // Pool start: every slot on the done list, marked unused.
 int launch_engine_init(const EngineBuffers& b, cudaStream_t st);
 // Publishes newly written pass descriptors: clamps the overshoot of `next` to the old total,

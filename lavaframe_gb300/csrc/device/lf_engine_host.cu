@@ -12,7 +12,6 @@ namespace lfrt
 namespace
 {
 constexpr int kDefaultSlots = 1 << 24;      // ~4.6 GB of path state (2^23 measured 2-3 % slower on C3)
-constexpr int kDefaultShadeCap = 512;       // shade kernel register cap (threads per SM)
 constexpr int kMaxJobs = 4096;
 constexpr size_t kRunRadianceBytes = size_t(2) << 30;   // radiance buffers of one frame run
 
@@ -85,6 +84,7 @@ lf_status engine_get(lf_ctx* c, EngineHost** out)
     A(&e->b.passDone, kPassRing);
     A(&e->b.ctl, 1);
     A(&e->ownCtr, 4);
+    A(&e->runPasses, kPassRing);
     if (err == cudaSuccess) err = cudaMallocHost((void**)&e->h_jobStage, sizeof(EngineJob) * kMaxJobs);
     if (err == cudaSuccess) err = cudaMallocHost((void**)&e->h_passStage, sizeof(EnginePass) * kPassRing);
     for (int k = 0; k < 2 && err == cudaSuccess; ++k)
@@ -354,12 +354,113 @@ lf_status engine_drain(EngineHost* e, unsigned long long* ctr, int maxDepth, int
 }
 
 // ------------------------------------------------------------------ frames on the engine
+namespace
+{
+// A frame run whose paths fit the engine's idle pool (launch_frame_run).
+lf_status frame_render_fitting(lf_frame* f, EngineHost* e, const Params& Pf, int firstSample, int count, long long paths)
+{
+    lf_ctx* c = f->ctx;
+    const bool tiledFrames = (f->flags & LF_FRAME_TILED_FRAMES) != 0;
+    const int tiles = f->numTilesX * f->numTilesY;
+    float4* arena = nullptr;
+    cudaError_t err = cudaMallocAsync((void**)&arena, sizeof(float4) * (size_t)paths, c->stream);
+    if (err != cudaSuccess) return cuda_fail(c, err, "pass radiance allocation");
+    std::vector<EnginePass> run;
+    unsigned long long base = 0;
+    for (int s = 0; s < count; s += f->sppBatch)
+    {
+        const int n = std::min(f->sppBatch, count - s);
+        for (int ty = f->numTilesY - 1; ty >= 0; --ty)
+            for (int tx = 0; tx < f->numTilesX; ++tx)
+            {
+                EnginePass q{};
+                q.firstSample = firstSample + s;
+                q.nSamples = n;
+                q.tileX = tx;
+                q.tileY = ty;
+                q.tileOrdinal = tiledFrames ? (f->numTilesY - 1 - ty) * f->numTilesX + tx : 0;
+                q.visW = std::min(Pf.tileW, f->W - tx * Pf.tileW);
+                q.visH = std::min(Pf.tileH, f->H - ty * Pf.tileH);
+                q.numPaths = (unsigned long long)n * q.visW * q.visH;
+                q.pathBase = base;
+                q.radiance = arena + base;
+                base += q.numPaths;
+                run.push_back(q);
+            }
+    }
+    if (run.size() > 1)
+    {
+        err = cudaMemcpyAsync(e->runPasses, run.data(), sizeof(EnginePass) * run.size(), cudaMemcpyHostToDevice, c->stream);
+        if (err != cudaSuccess)
+        {
+            cudaFreeAsync(arena, c->stream);
+            return cuda_fail(c, err, "pass table");
+        }
+    }
+    EngineJob one;
+    std::memset(&one, 0, sizeof one);
+    one.S = f->scene->view;
+    one.S.env.multiplier = Pf.hdrMultiplier;
+    one.P = Pf;
+    const bool sort = sort_on(e, &one);
+    if (sort)
+    {
+        lf_status st = ensure_sort_buckets(e);
+        if (st != LF_OK)
+        {
+            cudaFreeAsync(arena, c->stream);
+            return st;
+        }
+    }
+    EngineBuffers b = e->b;
+    b.ctr = f->bb.ctr;
+    b.sortByMaterial = sort ? 1 : 0;
+    int le = launch_frame_run(b, one, run[0], e->runPasses, (int)run.size(), (int)base, arena,
+                              (int)std::min<long long>(e->drainPaths, e->b.cap), c->stream);
+    if (le == 0)
+        le = run.size() == 1 ? launch_engine_accumulate(Pf, run[0], f->accum, f->accum64, c->stream)
+                             : launch_engine_accumulate_run(Pf, e->runPasses, (int)run.size() / tiles, f->numTilesX,
+                                                            f->numTilesY, f->accum, f->accum64, c->stream);
+    if (le == 0 && tiles == 1)
+    {
+        // the last pass stays readable (lf_frame_read_paths)
+        const EnginePass& last = run.back();
+        f->lastRadiance = arena;
+        f->lastRadianceSamples = last.nSamples;
+        if (run.size() > 1)
+        {
+            err = cudaMallocAsync((void**)&f->lastRadiance, sizeof(float4) * last.numPaths, c->stream);
+            if (err == cudaSuccess)
+                err = cudaMemcpyAsync(f->lastRadiance, last.radiance, sizeof(float4) * last.numPaths,
+                                      cudaMemcpyDeviceToDevice, c->stream);
+            cudaFreeAsync(arena, c->stream);
+            if (err != cudaSuccess) return cuda_fail(c, err, "pass radiance copy");
+        }
+    }
+    else
+        cudaFreeAsync(arena, c->stream);
+    return le ? cuda_fail(c, (cudaError_t)le, "direct run launch") : LF_OK;
+}
+}
+
 lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, int count)
 {
     lf_ctx* c = f->ctx;
     EngineHost* e = nullptr;
     lf_status st = engine_get(c, &e);
     if (st != LF_OK) return st;
+    if (f->lastRadiance)
+    {
+        cudaFreeAsync(f->lastRadiance, c->stream);
+        f->lastRadiance = nullptr;
+        f->lastRadianceSamples = 0;
+    }
+    // a run whose paths fit the idle pool
+    const long long paths = (long long)count * f->W * f->H;
+    const long long passes = (long long)((count + f->sppBatch - 1) / f->sppBatch) * f->numTilesX * f->numTilesY;
+    if (e->active == 0 && e->drainPaths > 0 && passes <= kPassRing && paths <= e->b.cap &&
+        (size_t)paths * sizeof(float4) <= kRunRadianceBytes)
+        return frame_render_fitting(f, e, Pf, firstSample, count, paths);
     if (f->engineJob < 0)
     {
         f->engineJob = engine_job_alloc(e, f->scene->view, Pf);
@@ -367,12 +468,6 @@ lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, in
     }
     else
         engine_job_write(e, f->engineJob, f->scene->view, Pf);
-    if (f->lastRadiance)
-    {
-        cudaFreeAsync(f->lastRadiance, c->stream);
-        f->lastRadiance = nullptr;
-        f->lastRadianceSamples = 0;
-    }
     const bool tiledFrames = (f->flags & LF_FRAME_TILED_FRAMES) != 0;
     const long long tilePix = (long long)Pf.tileW * Pf.tileH;
     // samples per pass: the frame's batch size, and below 2^31 paths per pass

@@ -14,6 +14,7 @@ struct EngineHost
     std::vector<void*> tables;   // job / pass tables, control block, counters
     size_t poolBytes = 0;
     unsigned long long* ownCtr = nullptr;   // counters of runs not tied to a frame
+    EnginePass* runPasses = nullptr;        // pass table of the runs on the idle pool
     EngineJob* h_jobStage = nullptr;        // pinned staging of the job table
     EnginePass* h_passStage = nullptr;      // pinned staging of the pass ring
     EngineCtl* h_ctl[2] = {nullptr, nullptr};

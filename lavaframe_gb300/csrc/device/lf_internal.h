@@ -29,7 +29,7 @@ struct lf_ctx
     cudaStream_t stream = nullptr;
     std::recursive_mutex mu;
     std::string err;
-    // status word of the kernels: in mapped page-locked memory, so that reading it after a
+    // status words of the kernels ([0]; [1] for lf_render_noalloc, which reports its own): in mapped page-locked memory, so that reading it after a
     // synchronisation needs no copy (the kernels only write it when something went wrong)
     volatile uint32_t* h_status = nullptr;
     uint32_t* d_status = nullptr;         // its device address

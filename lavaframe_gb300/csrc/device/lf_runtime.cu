@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "lf_engine.h"
 #include "lf_engine_host.h"
 #include "lf_pixel.h"
 
@@ -29,14 +30,14 @@ lf_status lf_ctx_create(int32_t device, lf_ctx** out)
     lf_ctx* c = new lf_ctx;
     c->device = device;
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaHostAlloc((void**)&c->h_status, sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
+        (e = cudaHostAlloc((void**)&c->h_status, 2 * sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
         (e = cudaHostGetDevicePointer((void**)&c->d_status, (void*)c->h_status, 0)) != cudaSuccess ||
         (e = cudaMalloc((void**)&c->d_stats, 3 * sizeof(unsigned long long))) != cudaSuccess)
     {
         delete c;
         return e == cudaErrorMemoryAllocation ? LF_ERR_OOM : LF_ERR_CUDA;
     }
-    *c->h_status = 0;
+    c->h_status[0] = c->h_status[1] = 0;
     cudaMemset(c->d_stats, 0, 3 * sizeof(unsigned long long));
     *out = c;
     return LF_OK;
@@ -1897,16 +1898,21 @@ namespace
 {
 constexpr long long kNoAllocPaths = 131072;   // path slots = max pixels of one tile
 constexpr size_t kNoAllocAlign = 256;
-constexpr size_t kNoAllocHeader = 256;        // queue sizes, status word, counters
+constexpr size_t kNoAllocHeader = 1024;       // control block, pass, counters
 constexpr size_t noalloc_round(size_t b) { return (b + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
-// PathSoA: o, d, T, L, A, rng, info, hit (16 B each), luv (8 B); two int queues; next-event records
-constexpr size_t kNoAllocBytes = kNoAllocHeader + 8 * noalloc_round(kNoAllocPaths * 16) +
-                                 noalloc_round(kNoAllocPaths * 8) + 2 * noalloc_round(kNoAllocPaths * 4) +
+// PathSoA: o, d, T, L, A, rng, info, hit and the radiance (16 B each), luv (8 B); two queues and the
+// split one (4 B each); next-event records
+constexpr size_t kNoAllocBytes = kNoAllocHeader + 9 * noalloc_round(kNoAllocPaths * 16) +
+                                 noalloc_round(kNoAllocPaths * 8) + 3 * noalloc_round(kNoAllocPaths * 4) +
                                  noalloc_round(kNoAllocPaths * sizeof(ShadowRec));
+// offsets in the header
+constexpr size_t kNoAllocCtl = 0, kNoAllocPass = 256, kNoAllocPassDone = 384, kNoAllocCtr = 512;
+static_assert(sizeof(EngineCtl) <= kNoAllocPass && sizeof(EnginePass) <= kNoAllocPassDone - kNoAllocPass,
+              "the header holds the control block and one pass");
 }
 
-// 30 MiB + 256 B (31.5 MB) on every GPU that loads the library, kept until the process exits.
-static_assert(kNoAllocBytes == 30ull * 1024 * 1024 + 256, "documented size of the no-alloc scratch array");
+// 32.5 MiB + 1 KiB (34.1 MB) on every GPU that loads the library, kept until the process exits.
+static_assert(kNoAllocBytes == 65ull * 512 * 1024 + 1024, "documented size of the no-alloc scratch array");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
 namespace
@@ -1960,32 +1966,39 @@ extern "C" lf_status lf_render_noalloc(lf_scene* sc, const lf_render_params* p, 
         return r;
     };
     const size_t N = (size_t)kNoAllocPaths;
-    PathSoA ps;
-    ps.o = (float4*)take(N * 16);
-    ps.d = (float4*)take(N * 16);
-    ps.T = (float4*)take(N * 16);
-    ps.L = (float4*)take(N * 16);
-    ps.A = (float4*)take(N * 16);
-    ps.rng = (uint4*)take(N * 16);
-    ps.info = (int4*)take(N * 16);
-    ps.hit = (float4*)take(N * 16);
-    ps.luv = (float2*)take(N * 8);
-    BounceBuffers bb;
-    bb.queue[0] = (int*)take(N * 4);
-    bb.queue[1] = (int*)take(N * 4);
-    bb.shadow = (ShadowRec*)take(N * sizeof(ShadowRec));
-    bb.count = (int*)(base + 0);
-    bb.shadowCount = (int*)(base + 8);
-    bb.status = (uint32_t*)(base + 12);
-    bb.ctr = (unsigned long long*)(base + 16);
-    bb.fetch = (unsigned long long*)(base + 48);
+    EngineBuffers b{};
+    b.ps.o = (float4*)take(N * 16);
+    b.ps.d = (float4*)take(N * 16);
+    b.ps.T = (float4*)take(N * 16);
+    b.ps.L = (float4*)take(N * 16);
+    b.ps.A = (float4*)take(N * 16);
+    b.ps.rng = (uint4*)take(N * 16);
+    b.ps.info = (int4*)take(N * 16);
+    b.ps.hit = (float4*)take(N * 16);
+    b.ps.luv = (float2*)take(N * 8);
+    float4* const radiance = (float4*)take(N * 16);
+    b.queue[0] = (int*)take(N * 4);
+    b.queue[1] = (int*)take(N * 4);
+    b.part = (int*)take(N * 4);
+    b.shadow = (ShadowRec*)take(N * sizeof(ShadowRec));
+    b.ctl = (EngineCtl*)(base + kNoAllocCtl);
+    EnginePass* const table = (EnginePass*)(base + kNoAllocPass);
+    b.passes = table;
+    b.passDone = (unsigned long long*)(base + kNoAllocPassDone);
+    b.ctr = (unsigned long long*)(base + kNoAllocCtr);
+    b.status = c->d_status + 1;
+    b.cap = (int)N;
+    b.shadeThreadsPerSm = kDefaultShadeCap;
 
-    // the array keeps the previous call's contents: clear sizes, status and counters
+    // the array keeps the previous call's contents: clear the counters
     cudaError_t e = cudaMemsetAsync(base, 0, kNoAllocHeader, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "no-alloc scratch clear");
 
-    ShadeScene Sv = sc->view;
-    Sv.env.multiplier = P.hdrMultiplier;
+    EngineJob one;
+    std::memset(&one, 0, sizeof one);
+    one.S = sc->view;
+    one.S.env.multiplier = P.hdrMultiplier;
+    one.P = P;
     const int numTilesX = (P.width + P.tileW - 1) / P.tileW, numTilesY = (P.height + P.tileH - 1) / P.tileH;
     const int spb = (int)std::max(1LL, std::min<long long>(64, kNoAllocPaths / tilePix));
     for (int s = 0; s < count;)
@@ -1994,22 +2007,26 @@ extern "C" lf_status lf_render_noalloc(lf_scene* sc, const lf_render_params* p, 
         for (int ty = numTilesY - 1; ty >= 0; --ty)
             for (int tx = 0; tx < numTilesX; ++tx)
             {
-                P.tileX = tx;
-                P.tileY = ty;
-                long long cap = (long long)n * tilePix;
-                cudaMemsetAsync(bb.count, 0, 2 * sizeof(int), c->stream);
-                int le = launch_generate(Sv, P, ps, first_sample + s, n, bb.queue[0], bb.count, c->stream);
-                for (int b = 0; le == 0 && b < P.maxDepth; ++b) le = launch_bounce(Sv, P, ps, bb, b, cap, c->stream);
-                if (le == 0) le = launch_accumulate(P, ps, n, (float4*)d_accum, nullptr, c->stream);
+                EnginePass q{};
+                q.firstSample = first_sample + s;
+                q.nSamples = n;
+                q.tileX = tx;
+                q.tileY = ty;
+                q.visW = std::min(P.tileW, P.width - tx * P.tileW);
+                q.visH = std::min(P.tileH, P.height - ty * P.tileH);
+                q.numPaths = (unsigned long long)n * q.visW * q.visH;
+                q.radiance = radiance;
+                int le = launch_frame_run(b, one, q, table, 1, (int)q.numPaths, radiance,
+                                          std::numeric_limits<int>::max(), c->stream);
+                if (le == 0) le = launch_engine_accumulate(P, q, (float4*)d_accum, nullptr, c->stream);
                 if (le) return cuda_fail(c, (cudaError_t)le, "no-alloc render launch");
             }
         s += n;
     }
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "no-alloc render");
-    uint32_t bits = 0;
-    e = cudaMemcpy(&bits, bb.status, sizeof bits, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(c, e, "no-alloc status readback");
+    const uint32_t bits = c->h_status[1];
+    c->h_status[1] = 0;
     if (bits)
     {
         c->devErrors |= bits;
