@@ -105,14 +105,6 @@ lf_status engine_get(lf_ctx* c, EngineHost** out)
     e->b.shadeThreadsPerSm = kDefaultShadeCap;
     e->jobUsed.assign(kMaxJobs, 0);
     e->jobGen.assign(kMaxJobs, 0);
-    // pass radiance buffers come from the stream-ordered pool; keep up to 8 GB of it cached
-    // between runs instead of handing it back to CUDA at every synchronisation
-    cudaMemPool_t pool = nullptr;
-    if (cudaDeviceGetDefaultMemPool(&pool, c->device) == cudaSuccess)
-    {
-        uint64_t keep = uint64_t(8) << 30;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
     cudaMemsetAsync(e->b.ctl, 0, sizeof(EngineCtl), c->stream);
     cudaMemsetAsync(e->b.passDone, 0, sizeof(unsigned long long) * kPassRing, c->stream);
     cudaMemsetAsync(e->ownCtr, 0, 4 * sizeof(unsigned long long), c->stream);

@@ -352,6 +352,24 @@ __global__ void __launch_bounds__(kWarps * 32) guide_train_kernel(Net net, const
         if (S.dW[i] != 0.f) atomicAdd(&gW[i], S.dW[i]);
 }
 
+// out = grad * scale, and grad cleared: the gradients of a host query leave the accumulators ready for
+// the next pass (weights, then grid, then the loss; counts of floats, multiples of 4 but the loss).
+__global__ void guide_scale_kernel(float* gW, float* gGrid, float* loss, float scale, float* out)
+{
+    constexpr int nW = kWeights / 4, nG = kGridParams / 4;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nW + nG) return;
+    float4* g = i < nW ? reinterpret_cast<float4*>(gW) + i : reinterpret_cast<float4*>(gGrid) + (i - nW);
+    const float4 v = *g;
+    *g = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(out)[i] = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+    if (i == 0)
+    {
+        out[kWeights + kGridParams] = *loss * scale;
+        *loss = 0.f;
+    }
+}
+
 // Adam over FP32 master parameters (gradients scaled by gradScale, then cleared), refreshing
 // the FP16 working copy.
 __global__ void guide_adam_kernel(float* master, __half* work, float* m, float* v, float* grad, int n, float lr,
@@ -685,25 +703,21 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats);
+    constexpr size_t outs = kWeights + kGridParams + 1;
+    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats + outs);
     if (st != LF_OK) return st;
+    float* const out = gd->scratch + (size_t)n * kSampleFloats;   // samples are 16 floats: aligned
     cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-    cudaMemsetAsync(gd->wGrad, 0, kWeights * sizeof(float), c->stream);
-    cudaMemsetAsync(gd->gGrad, 0, (size_t)kGridParams * sizeof(float), c->stream);
-    cudaMemsetAsync(gd->dLoss, 0, sizeof(float), c->stream);
+    cudaMemsetAsync(gd->dLoss, 0, sizeof(float), c->stream);      // training steps leave theirs
     st = run_gradients(gd, gd->scratch, n);
     if (st != LF_OK) return st;
-    cudaMemcpyAsync(dweights, gd->wGrad, kWeights * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(dgrid, gd->gGrad, (size_t)kGridParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(loss, gd->dLoss, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemsetAsync(gd->wGrad, 0, kWeights * sizeof(float), c->stream);
-    cudaMemsetAsync(gd->gGrad, 0, (size_t)kGridParams * sizeof(float), c->stream);
+    guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(gd->wGrad, gd->gGrad, gd->dLoss,
+                                                                                      1.f / (float)n, out);
+    cudaMemcpyAsync(dweights, out, kWeights * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(dgrid, out + kWeights, (size_t)kGridParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(loss, out + kWeights + kGridParams, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide gradients");
-    const float inv = 1.f / (float)n;
-    for (int i = 0; i < kWeights; ++i) dweights[i] *= inv;
-    for (int i = 0; i < kGridParams; ++i) dgrid[i] *= inv;
-    *loss *= inv;
     return check_device(c);
 }
 

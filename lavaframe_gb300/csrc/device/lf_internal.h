@@ -187,6 +187,11 @@ inline lf_status check_device(lf_ctx* c)
 // whole frame unless the parameters set a tile size.
 void fill_params(Params& P, const lf_render_params* p, const lf_scene* sc);
 
+// The copy streams and events of calls that overlap copies with kernels, made on first use.
+cudaError_t ensure_chunk_streams(lf_ctx* c);
+// The colour channels of n padded pixels into host memory, after the stream's work (synchronises).
+cudaError_t copy_rgb(lf_ctx* c, const float4* src, size_t n, float* rgb);
+
 struct RefNode
 {
     float bmin[3], bmax[3], lr[3];

@@ -170,6 +170,29 @@ __global__ void accumulate_kernel(Params P, PathSoA ps, int nSamples, float4* ac
     }
 }
 
+// Four pixels a thread: 64 bytes read, 48 written, in 16-byte words (HBM-bound; the copy to the
+// host that follows takes several times longer).
+__global__ void pack_rgb_kernel(const float4* src, long long n, float* dst)
+{
+    const long long groups = n >> 2;
+    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += (long long)gridDim.x * blockDim.x)
+    {
+        const float4 a = src[4 * g], b = src[4 * g + 1], c = src[4 * g + 2], d = src[4 * g + 3];
+        float4* o = reinterpret_cast<float4*>(dst + 12 * g);
+        o[0] = make_float4(a.x, a.y, a.z, b.x);
+        o[1] = make_float4(b.y, b.z, c.x, c.y);
+        o[2] = make_float4(c.z, d.x, d.y, d.z);
+    }
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3))
+    {
+        const long long i = (groups << 2) + threadIdx.x;
+        const float4 a = src[i];
+        dst[3 * i] = a.x;
+        dst[3 * i + 1] = a.y;
+        dst[3 * i + 2] = a.z;
+    }
+}
+
 // ------------------------------------------------------------------ ray queries
 template <bool kStats>
 __global__ void trace_closest_kernel(DevScene S, const float4* rays, long long n, int4* hits, int lights,
@@ -465,6 +488,13 @@ int launch_accumulate(const Params& P, const PathSoA& ps, int nSamples, float4* 
     const int B = 256;
     int g = grid_for((const void*)accumulate_kernel, B, (long long)P.tileW * P.tileH);
     accumulate_kernel<<<g, B, 0, st>>>(P, ps, nSamples, accum, accum64);
+    return (int)cudaGetLastError();
+}
+
+int launch_pack_rgb(const float4* src, long long n, float* dst, cudaStream_t st)
+{
+    const int B = 256;
+    pack_rgb_kernel<<<grid_for((const void*)pack_rgb_kernel, B, (n >> 2) + 4), B, 0, st>>>(src, n, dst);
     return (int)cudaGetLastError();
 }
 

@@ -78,6 +78,8 @@ int launch_bounce(const ShadeScene& S, const Params& P, const PathSoA& ps, const
                   long long cap, cudaStream_t st);
 int launch_accumulate(const Params& P, const PathSoA& ps, int nSamples, float4* accum, double* accum64,
                       cudaStream_t st);
+// n float4 -> 3 n floats (the w components are dropped).
+int launch_pack_rgb(const float4* src, long long n, float* dst, cudaStream_t st);
 int launch_trace_closest(const DevScene& S, const float4* rays, long long n, int4* hits, int lights, bool stats,
                          uint32_t* status, unsigned long long* stat3, cudaStream_t st);
 // `next`: two counters, zero before the first launch and left at zero by every launch.

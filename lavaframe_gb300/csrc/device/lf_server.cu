@@ -495,20 +495,11 @@ lf_status lf_server_read(lf_server* s, int64_t job_id, float* rgb)
     if (it == s->jobs.end()) return LF_ERR_INVALID;
     ServerJob& j = it->second;
     if (j.state != LF_JOB_DONE) return fail(s->ctx, LF_ERR_STATE, "job not done");
-    std::vector<float4> tmp((size_t)j.params.width * j.params.height);
     lf_ctx* c = s->ctx;
     std::lock_guard<std::recursive_mutex> g(c->mu);
     cudaSetDevice(c->device);
-    cudaError_t e = cudaMemcpyAsync(tmp.data(), j.accum, tmp.size() * sizeof(float4), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "job readback");
-    for (size_t i = 0; i < tmp.size(); ++i)
-    {
-        rgb[i * 3 + 0] = tmp[i].x;
-        rgb[i * 3 + 1] = tmp[i].y;
-        rgb[i * 3 + 2] = tmp[i].z;
-    }
-    return LF_OK;
+    const cudaError_t e = copy_rgb(c, j.accum, (size_t)j.params.width * j.params.height, rgb);
+    return e == cudaSuccess ? LF_OK : cuda_fail(c, e, "job readback");
 }
 
 lf_status lf_server_release_job(lf_server* s, int64_t job_id)

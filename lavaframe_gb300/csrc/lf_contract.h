@@ -28,10 +28,14 @@
 
 // The transcendental functions (LF_HD_CALL) stay out of line on the device: the shading kernel
 // calls them from many places and inlining every copy costs more in instruction fetch than the
-// calls do.
+// calls do. A translation unit of small kernels defines LF_CONTRACT_INLINE to have them inline.
 #if defined(__CUDACC__)
 #define LF_HD __host__ __device__ __forceinline__
+#if defined(LF_CONTRACT_INLINE)
+#define LF_HD_CALL LF_HD
+#else
 #define LF_HD_CALL [[maybe_unused]] static __host__ __device__ __noinline__
+#endif
 #else
 #define LF_HD inline
 #define LF_HD_CALL inline
