@@ -325,7 +325,14 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
     {
         const int q = tile * kTcRows + row;
         const bool valid = q < n;
-        encode_row_direct(net, queries + (size_t)(valid ? q : 0) * kSampleFloats, valid, sA, row);
+        {
+            // position, outgoing direction and normal in three 16-byte loads (records are 64 bytes apart)
+            float rec[12];
+            const float4* src = reinterpret_cast<const float4*>(queries + (size_t)(valid ? q : 0) * kSampleFloats);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) *reinterpret_cast<float4*>(rec + 4 * k) = src[k];
+            encode_row_direct(net, rec, valid, sA, row);
+        }
         for (int layer = 0; layer < 4; ++layer)
         {
             // the group's A tile (and, from layer 1, its reads of the accumulator) are complete
@@ -385,23 +392,35 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
         const float invEs = 1.f / es;
         float* dst = mix + (size_t)(valid ? q : 0) * kMixFloats;
         float cum = 0.f;
+        // four lobes at a time: 20 values in five 16-byte stores
 #pragma unroll
-        for (int i = 0; i < kLobes; ++i)
+        for (int half = 0; half < kLobes; half += 4)
         {
-            float o5[4], mu[3], k;
+            float o[20];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o5[j] = tmem_ld1(acc + lane0 + 5 * i + j);
-            tmem_wait_ld();
-            lobe_params(o5, mu, &k);
-            cum += e[i] * invEs;
-            if (valid)
+            for (int i = 0; i < 4; ++i)
             {
-                dst[5 * i + 0] = mu[0];
-                dst[5 * i + 1] = mu[1];
-                dst[5 * i + 2] = mu[2];
-                dst[5 * i + 3] = k;
-                dst[5 * i + 4] = i == kLobes - 1 ? 1.f : cum;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[5 * i + j] = tmem_ld1(acc + lane0 + 5 * (half + i) + j);
             }
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                float mu[3], k;
+                lobe_params(o + 5 * i, mu, &k);
+                cum += e[half + i] * invEs;
+                o[5 * i + 0] = mu[0];
+                o[5 * i + 1] = mu[1];
+                o[5 * i + 2] = mu[2];
+                o[5 * i + 3] = k;
+                o[5 * i + 4] = half + i == kLobes - 1 ? 1.f : cum;
+            }
+            if (valid)
+#pragma unroll
+                for (int k = 0; k < 5; ++k)
+                    *reinterpret_cast<float4*>(dst + 5 * half + 4 * k) =
+                        make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
         }
     }
     fence_before_sync();

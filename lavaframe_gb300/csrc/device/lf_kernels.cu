@@ -57,22 +57,17 @@ __global__ void generate_kernel(ShadeScene S, Params P, PathSoA ps, int firstSam
 }
 
 // ------------------------------------------------------------------ extend
-// Warps take queue entries 32 at a time from `fetch`; 72 registers (7 blocks of 128 per SM).
+// 72 registers (7 blocks of 128 per SM).
 __global__ void __maxnreg__(72) extend_kernel(ShadeScene S, Params P, PathSoA ps, const int* queue, const int* qcount,
-                                              unsigned long long* fetch, uint32_t* status, unsigned long long* ctr)
+                                              int* fetch, uint32_t* status, unsigned long long* ctr)
 {
     const int n = *qcount;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr[1], (unsigned long long)n);
     const bool lights = P.useLights != 0;
-    const int lane = threadIdx.x & 31;
-    while (true)
+    for (QueueShare share(n); share.more(); share.next(fetch))
     {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(fetch, 32ull);
-        base = __shfl_sync(kFull, base, 0);
-        if (base >= (unsigned long long)n) break;
-        const int i = (int)base + lane;
-        if (i >= n) continue;
+        const int i = share.entry();
+        if (i < 0) continue;
         int p = queue[i];
         float4 o4 = ps.o[p], d4 = ps.d[p];
         Hit h;
@@ -91,17 +86,13 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(ShadeScene S, Params P, P
                                                         int* sqCount, int cap, uint32_t* status,
                                                         unsigned long long* ctr)
 {
-    const int n = *qinCount;
-    const int stride = gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    const int warpBase = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-    for (int base = warpBase; base < n; base += stride)
+    for (QueueShare share(*qinCount); share.more(); share.next())
     {
-        int i = base + lane;
+        const int i = share.entry();
         bool pushExt = false, pushShadow = false;
         int p = -1;
         ShadowRec rec;
-        if (i < n)
+        if (i >= 0)
         {
             p = qin[i];
             shade_path<kLights>(S, P, ps, p, ctr, pushExt, pushShadow, rec);
@@ -113,20 +104,15 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(ShadeScene S, Params P, P
 
 // ------------------------------------------------------------------ shadow
 __global__ void __maxnreg__(72) shadow_kernel(ShadeScene S, Params P, PathSoA ps, const ShadowRec* sq,
-                                              const int* sqCount, unsigned long long* fetch, uint32_t* status,
+                                              const int* sqCount, int* fetch, uint32_t* status,
                                               unsigned long long* ctr)
 {
-    const int n = *sqCount;
     unsigned long long rays = 0;
-    const int lane = threadIdx.x & 31;
-    while (true)
+    for (QueueShare share(*sqCount); share.more(); share.next(fetch))
     {
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(fetch, 32ull);
-        base = __shfl_sync(kFull, base, 0);
-        if (base >= (unsigned long long)n) break;
-        const int i = (int)base + lane;
-        if (i < n) set_error(status, shadow_path(S, P, ps, sq + i, rays));
+        const int i = share.entry();
+        if (i >= 0) set_error(status, shadow_path(S, P, ps, sq + i, rays));
+        __syncwarp();
     }
     warp_count_add(&ctr[2], rays);
 }
@@ -253,7 +239,7 @@ __global__ void guide_query_kernel(ShadeScene S, PathSoA ps, const int* queue, c
         if (pixelShare > 0 && p >= pixelShare) continue;
         const float4 h = ps.hit[p];
         float* q = queries + (size_t)(pixelShare > 0 ? p : i) * guide::kSampleFloats;
-        float v[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 1.f};
+        float v[12] = {0.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
         const int prim = __float_as_int(h.z), light = __float_as_int(h.w);
         if (h.x != kInfinity && light < 0 && prim >= 0)
         {
@@ -262,7 +248,8 @@ __global__ void guide_query_kernel(ShadeScene S, PathSoA ps, const int* queue, c
             const float vv[9] = {g.fhp.x, g.fhp.y, g.fhp.z, -d4.x, -d4.y, -d4.z, g.nrm.x, g.nrm.y, g.nrm.z};
             for (int k = 0; k < 9; ++k) v[k] = vv[k];
         }
-        for (int k = 0; k < 9; ++k) q[k] = v[k];
+        for (int k = 0; k < 3; ++k)   // 16-byte stores: the records of a warp are 64 bytes apart
+            reinterpret_cast<float4*>(q)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     }
 }
 
@@ -273,17 +260,13 @@ __global__ void __launch_bounds__(128, 4) shade_guided_kernel(ShadeScene S, Para
                                                                ShadowRec* sq, int* sqCount, int cap, uint32_t* status,
                                                                unsigned long long* ctr, GuideCtx gc, int pixelShare)
 {
-    const int n = *qinCount;
-    const int stride = gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    const int warpBase = (blockIdx.x * blockDim.x + threadIdx.x) & ~31;
-    for (int base = warpBase; base < n; base += stride)
+    for (QueueShare share(*qinCount); share.more(); share.next())
     {
-        int i = base + lane;
+        const int i = share.entry();
         bool pushExt = false, pushShadow = false;
         int p = -1;
         ShadowRec rec;
-        if (i < n)
+        if (i >= 0)
         {
             p = qin[i];
             shade_path_t<true>(S, P, ps, p, ctr, pushExt, pushShadow, rec, gc, pixelShare > 0 ? p % pixelShare : i);
@@ -413,33 +396,41 @@ int launch_generate(const ShadeScene& S, const Params& P, const PathSoA& ps, int
     return (int)cudaGetLastError();
 }
 
+namespace
+{
+// The counters a bounce fills: its output queue's, the next-event records' and the work counters (all
+// but its input queue's, which is the first or the last of the array).
+void clear_bounce(const BounceBuffers& b, int bounce, cudaStream_t st)
+{
+    cudaMemsetAsync(b.counters + ((bounce & 1) ? 0 : 1), 0, 4 * sizeof(int), st);
+}
+}
+
 int launch_bounce(const ShadeScene& S, const Params& P, const PathSoA& ps, const BounceBuffers& b, int bounce,
                   long long cap, cudaStream_t st)
 {
     int* qin = b.queue[bounce & 1];
     int* qout = b.queue[(bounce + 1) & 1];
-    int* cin = b.count + (bounce & 1);
-    int* cout = b.count + ((bounce + 1) & 1);
-    cudaMemsetAsync(cout, 0, sizeof(int), st);
-    cudaMemsetAsync(b.shadowCount, 0, sizeof(int), st);
+    const int *cin = b.count(bounce & 1), *shadowCount = b.counters + 3;
+    int* cout = b.count((bounce + 1) & 1);
+    clear_bounce(b, bounce, st);
     const int BE = 128, BS = 128, BW = 128;
-    cudaMemsetAsync(b.fetch, 0, 2 * sizeof(unsigned long long), st);
-    int ge = grid_for((const void*)extend_kernel, BE, cap);
-    extend_kernel<<<ge, BE, 0, st>>>(S, P, ps, qin, cin, b.fetch, b.status, b.ctr);
+    int ge = grid_for((const void*)extend_kernel, BE, 32 * cap);
+    extend_kernel<<<ge, BE, 0, st>>>(S, P, ps, qin, cin, b.counters + 1, b.status, b.ctr);
     if (P.useLights)
     {
-        int gs = grid_for((const void*)shade_kernel<true>, BS, cap);
-        shade_kernel<true><<<gs, BS, 0, st>>>(S, P, ps, qin, cin, qout, cout, b.shadow, b.shadowCount, (int)cap, b.status,
+        int gs = grid_for((const void*)shade_kernel<true>, BS, 32 * cap);
+        shade_kernel<true><<<gs, BS, 0, st>>>(S, P, ps, qin, cin, qout, cout, b.shadow, b.counters + 3, (int)cap, b.status,
                                               b.ctr);
     }
     else
     {
-        int gs = grid_for((const void*)shade_kernel<false>, BS, cap);
-        shade_kernel<false><<<gs, BS, 0, st>>>(S, P, ps, qin, cin, qout, cout, b.shadow, b.shadowCount, (int)cap,
+        int gs = grid_for((const void*)shade_kernel<false>, BS, 32 * cap);
+        shade_kernel<false><<<gs, BS, 0, st>>>(S, P, ps, qin, cin, qout, cout, b.shadow, b.counters + 3, (int)cap,
                                                b.status, b.ctr);
     }
-    int gw = grid_for((const void*)shadow_kernel, BW, cap);
-    shadow_kernel<<<gw, BW, 0, st>>>(S, P, ps, b.shadow, b.shadowCount, b.fetch + 1, b.status, b.ctr);
+    int gw = grid_for((const void*)shadow_kernel, BW, 32 * cap);
+    shadow_kernel<<<gw, BW, 0, st>>>(S, P, ps, b.shadow, shadowCount, b.counters + 2, b.status, b.ctr);
     return (int)cudaGetLastError();
 }
 
@@ -448,13 +439,11 @@ int launch_bounce_guided(const ShadeScene& S, const Params& P, const PathSoA& ps
 {
     int* qin = b.queue[bounce & 1];
     int* qout = b.queue[(bounce + 1) & 1];
-    int* cin = b.count + (bounce & 1);
-    int* cout = b.count + ((bounce + 1) & 1);
-    cudaMemsetAsync(cout, 0, sizeof(int), st);
-    cudaMemsetAsync(b.shadowCount, 0, sizeof(int), st);
+    const int *cin = b.count(bounce & 1), *shadowCount = b.counters + 3;
+    int* cout = b.count((bounce + 1) & 1);
+    clear_bounce(b, bounce, st);
     const int B = 128;
-    cudaMemsetAsync(b.fetch, 0, 2 * sizeof(unsigned long long), st);
-    extend_kernel<<<grid_for((const void*)extend_kernel, B, cap), B, 0, st>>>(S, P, ps, qin, cin, b.fetch, b.status,
+    extend_kernel<<<grid_for((const void*)extend_kernel, B, 32 * cap), B, 0, st>>>(S, P, ps, qin, cin, b.counters + 1, b.status,
                                                                               b.ctr);
     // First bounce of a batch of several samples: the samples of a pixel hit its footprint
     // from the same camera, so they share one mixture, inferred from the pixel's sample-0 path
@@ -469,10 +458,10 @@ int launch_bounce_guided(const ShadeScene& S, const Params& P, const PathSoA& ps
                          : guide::launch_infer(g.net, g.queries, nq, qcap, g.mix, st);
     if (e) return e;
     GuideCtx gc{g.mix, g.rec, g.alpha, g.maxDepth, cap};
-    shade_guided_kernel<<<grid_for((const void*)shade_guided_kernel, B, cap), B, 0, st>>>(
-        S, P, ps, qin, cin, qout, cout, b.shadow, b.shadowCount, (int)cap, b.status, b.ctr, gc, share);
-    shadow_kernel<<<grid_for((const void*)shadow_kernel, B, cap), B, 0, st>>>(S, P, ps, b.shadow, b.shadowCount,
-                                                                             b.fetch + 1, b.status, b.ctr);
+    shade_guided_kernel<<<grid_for((const void*)shade_guided_kernel, B, 32 * cap), B, 0, st>>>(
+        S, P, ps, qin, cin, qout, cout, b.shadow, b.counters + 3, (int)cap, b.status, b.ctr, gc, share);
+    shadow_kernel<<<grid_for((const void*)shadow_kernel, B, 32 * cap), B, 0, st>>>(S, P, ps, b.shadow, shadowCount,
+                                                                             b.counters + 2, b.status, b.ctr);
     return (int)cudaGetLastError();
 }
 

@@ -35,12 +35,15 @@ struct ShadowRec
 struct BounceBuffers
 {
     int* queue[2];
-    int* count;          // [2] queue sizes
+    // counters in one array, so that a bounce clears its own with one memset whatever its parity:
+    // [0] size of queue 0, [1], [2] work counters of the extend / shadow kernels, [3] next-event
+    // records, [4] size of queue 1
+    int* counters;
     ShadowRec* shadow;
-    int* shadowCount;
     uint32_t* status;
     unsigned long long* ctr;   // [0] paths, [1] extension rays, [2] shadow rays, [3] light clamps
-    unsigned long long* fetch; // [2] work counters of the extend / shadow kernels
+
+    __host__ __device__ int* count(int queue) const { return counters + 4 * queue; }
 };
 
 // Floats per recorded path vertex of guided rendering (see GuideCtx in lf_pathops.cuh).

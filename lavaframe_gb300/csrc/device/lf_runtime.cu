@@ -1387,10 +1387,8 @@ lf_status alloc_paths(lf_frame* f, long long cap)
     A(&f->ps.hit, cap);
     A(&f->bb.queue[0], cap);
     A(&f->bb.queue[1], cap);
-    A(&f->bb.count, 2);
+    A(&f->bb.counters, 5);
     A(&f->bb.shadow, cap);
-    A(&f->bb.shadowCount, 1);
-    A(&f->bb.fetch, 2);
     if (e != cudaSuccess)
     {
         free_frame_buffers(f);
@@ -1521,8 +1519,8 @@ lf_status run_batch(lf_frame* f, Params P, int firstSample, int n, bool record =
         cudaError_t ce = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
         if (ce != cudaSuccess) return cuda_fail(c, ce, "batch graph capture");
     }
-    cudaMemsetAsync(f->bb.count, 0, 2 * sizeof(int), c->stream);
-    int e = launch_generate(Sv, P, f->ps, firstSample, n, f->bb.queue[0], f->bb.count, c->stream);
+    cudaMemsetAsync(f->bb.counters, 0, 5 * sizeof(int), c->stream);
+    int e = launch_generate(Sv, P, f->ps, firstSample, n, f->bb.queue[0], f->bb.count(0), c->stream);
     if (e) return graph ? end_batch_graph(f, cudaErrorLaunchFailure, "generate launch")
                         : cuda_fail(c, (cudaError_t)e, "generate launch");
     BounceBuffers bb = f->bb;
