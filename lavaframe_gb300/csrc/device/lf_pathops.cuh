@@ -163,9 +163,8 @@ __device__ __forceinline__ void gen_path(const Params& P, int tileX, int tileY, 
     jx = jx / ((float)P.width * 0.5f);
     jy = jy / ((float)P.height * 0.5f);
     float dx = ctx + jx, dy = cty + jy;
-    float scale = lfc::tan_c(P.fov * 0.5f);
-    dy = dy * ((float)P.height / (float)P.width * scale);
-    dx = dx * scale;
+    dy = dy * P.scaleY;
+    dx = dx * P.scaleX;
     v3 right(P.cam_right[0], P.cam_right[1], P.cam_right[2]);
     v3 up(P.cam_up[0], P.cam_up[1], P.cam_up[2]);
     v3 fwd(P.cam_fwd[0], P.cam_fwd[1], P.cam_fwd[2]);
@@ -329,7 +328,8 @@ __device__ __forceinline__ void shade_path_t(const ShadeScene& S, const Params& 
 
         if (lfc::dot(s.normal, s.ffnormal) > 0.0f) A = v3(0.0f);
         L = L + s.mat.emission * T;
-        T = T * lfc::vexp(-A * t);
+        // no absorption: exp(-0) = 1 in every channel
+        if (A.x != 0.0f || A.y != 0.0f || A.z != 0.0f) T = T * lfc::vexp(-A * t);
 
         // ---- DirectLight (pathtrace.glsl:126-204): candidates, visibility later
         BsdfCtx bc{s.eta, s.mat, s.tangent, s.bitangent};

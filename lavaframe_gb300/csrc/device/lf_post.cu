@@ -25,6 +25,7 @@ struct PostParams
 
 __device__ __forceinline__ int wrapi(int i, int n)
 {
+    if ((unsigned)i < (unsigned)n) return i;
     int r = i % n;
     return r < 0 ? r + n : r;
 }

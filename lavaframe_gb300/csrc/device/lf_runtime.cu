@@ -1346,7 +1346,8 @@ void fill_params(Params& P, const lf_render_params* p, const lf_scene* sc)
         P.cam_up[k] = p->cam_up[k];
         P.cam_fwd[k] = p->cam_forward[k];
     }
-    P.fov = p->cam_fov;
+    P.scaleX = lfc::tan_c(p->cam_fov * 0.5f);
+    P.scaleY = (float)p->height / (float)p->width * P.scaleX;
     P.focalDist = p->cam_focal_dist;
     P.aperture = p->cam_aperture;
     P.seed = p->seed;

