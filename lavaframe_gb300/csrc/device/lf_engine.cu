@@ -412,8 +412,9 @@ __global__ void __launch_bounds__(kRefillBlock) engine_refill_kernel(EngineBuffe
 }
 
 // ------------------------------------------------------------------ extend / shade / shadow
-// The traversal kernels are held to 72 registers (7 blocks of 128 threads per SM; a few spills)
-// whatever block size they are launched with.
+// The traversal kernels are held to 72 (closest hit) and 64 registers (occlusion): 7 and 8 blocks of
+// 128 threads per SM, a few spills, whatever block size they are launched with. Spheres 1080p x 8
+// 13.01 ms; both at 72 13.11, both at 64 13.08, 80 and 80 13.6, 72 and 56 13.06.
 template <bool kOne>
 __global__ void __maxnreg__(72) engine_extend_kernel(EngineBuffers b, EngineJob one, int parity)
 {
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(256, kThreadsPerSm ? kThreadsPerSm / 256 : 1)
 }
 
 template <bool kOne>
-__global__ void __maxnreg__(72) engine_shadow_kernel(EngineBuffers b, EngineJob one, int parity)
+__global__ void __maxnreg__(64) engine_shadow_kernel(EngineBuffers b, EngineJob one, int parity)
 {
     __shared__ BlockDone bd;
     block_done_begin(bd);

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(ShadeScene S, Params P, P
 }
 
 // ------------------------------------------------------------------ shadow
-__global__ void __maxnreg__(72) shadow_kernel(ShadeScene S, Params P, PathSoA ps, const ShadowRec* sq,
+__global__ void __maxnreg__(64) shadow_kernel(ShadeScene S, Params P, PathSoA ps, const ShadowRec* sq,
                                               const int* sqCount, int* fetch, uint32_t* status,
                                               unsigned long long* ctr)
 {

@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(DevScene S, const
 // launch. (Refilling single lanes as their rays end, with the traversal state kept in registers,
 // measured 35 % slower: the binned rays of a warp stop sharing nodes and the refill logic spills.)
 template <bool kAny>
-__global__ void __launch_bounds__(128) trace_fetch_wide_kernel(DevScene S, const float4* rays, const int* perm,
+__global__ void __launch_bounds__(128, kAny ? 8 : 7) trace_fetch_wide_kernel(DevScene S, const float4* rays, const int* perm,
                                                                long long n, int4* hits, uint8_t* occluded, int lights,
                                                                unsigned long long* next, uint32_t* status, int chunk)
 {
