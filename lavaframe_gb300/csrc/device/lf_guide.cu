@@ -218,7 +218,7 @@ __device__ __forceinline__ void encode_tile(const Net& net, const float* p, cons
 // One pass over n training samples: adds the per-sample gradients (not divided by n) of every
 // weight into gW and of every grid parameter into gGrid, and the summed loss into loss.
 __global__ void __launch_bounds__(kWarps * 32) guide_train_kernel(Net net, const float* samples, int n, float* gW,
-                                                                  float* gGrid, float* loss)
+                                                                  float* gGrid, double* loss)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SharedTrain& S = *reinterpret_cast<SharedTrain*>(smem_raw);
@@ -346,15 +346,16 @@ __global__ void __launch_bounds__(kWarps * 32) guide_train_kernel(Net net, const
         __syncwarp();
     }
     for (int off = 16; off > 0; off >>= 1) lossSum += __shfl_xor_sync(kFull, lossSum, off);
-    if (lane == 0 && lossSum != 0.f) atomicAdd(loss, lossSum);
+    if (lane == 0 && lossSum != 0.f) atomicAdd(loss, (double)lossSum);
     __syncthreads();
     for (int i = threadIdx.x; i < kWeights; i += blockDim.x)
         if (S.dW[i] != 0.f) atomicAdd(&gW[i], S.dW[i]);
 }
 
-// out = grad * scale, and grad cleared: the gradients of a host query leave the accumulators ready for
-// the next pass (weights, then grid, then the loss; counts of floats, multiples of 4 but the loss).
-__global__ void guide_scale_kernel(float* gW, float* gGrid, float* loss, float scale, float* out)
+// The gradients times scale (weights to outW, grid to outGrid, the loss to outLoss), and their
+// accumulators cleared: a host query leaves them ready for the next pass.
+__global__ void guide_scale_kernel(float* gW, float* gGrid, double* loss, float scale, float* outW, float* outGrid,
+                                   float* outLoss)
 {
     constexpr int nW = kWeights / 4, nG = kGridParams / 4;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -362,11 +363,12 @@ __global__ void guide_scale_kernel(float* gW, float* gGrid, float* loss, float s
     float4* g = i < nW ? reinterpret_cast<float4*>(gW) + i : reinterpret_cast<float4*>(gGrid) + (i - nW);
     const float4 v = *g;
     *g = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4*>(out)[i] = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+    float4* o = i < nW ? reinterpret_cast<float4*>(outW) + i : reinterpret_cast<float4*>(outGrid) + (i - nW);
+    *o = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
     if (i == 0)
     {
-        out[kWeights + kGridParams] = *loss * scale;
-        *loss = 0.f;
+        *outLoss = (float)(*loss * (double)scale);
+        *loss = 0.0;
     }
 }
 
@@ -515,7 +517,7 @@ struct lf_guide
     float* gM = nullptr;
     float* gV = nullptr;
     float* gGrad = nullptr;
-    float* dLoss = nullptr;
+    double* dLoss = nullptr;        // summed in double: 32-bit sums of a batch differed by 1e-6 from run to run
     float* scratch = nullptr;       // device samples of the host-buffer entry points
     size_t scratchFloats = 0;
     Net net{};
@@ -638,7 +640,7 @@ lf_status lf_guide_create(lf_ctx* c, const float scene_lo[3], const float scene_
     to_half_kernel<<<grid_blocks(kGridParams, 256), 256, 0, c->stream>>>(gd->gMaster, gd->gWork, kGridParams);
     for (float* p : {gd->wM, gd->wV, gd->wGrad}) cudaMemsetAsync(p, 0, kWeights * sizeof(float), c->stream);
     for (float* p : {gd->gM, gd->gV, gd->gGrad}) cudaMemsetAsync(p, 0, (size_t)kGridParams * sizeof(float), c->stream);
-    cudaMemsetAsync(gd->dLoss, 0, sizeof(float), c->stream);
+    cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);
     gd->net.W = gd->wWork;
     gd->net.grid = gd->gWork;
     res_levels(gd->net.res);
@@ -703,21 +705,25 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    constexpr size_t outs = kWeights + kGridParams + 1;
-    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats + outs);
+    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats + kGridParams);
     if (st != LF_OK) return st;
-    float* const out = gd->scratch + (size_t)n * kSampleFloats;   // samples are 16 floats: aligned
+    if (!ensure_stage(c)) return fail(c, LF_ERR_OOM, "guide gradient staging");
+    float* const outGrid = gd->scratch + (size_t)n * kSampleFloats;   // samples are 16 floats: aligned
+    // the small results go to page-locked memory, which saves two copies' latencies
+    static_assert((kWeights + 1) * sizeof(float) <= kStageBytes, "weight gradients and the loss fit the staging block");
+    float* const hW = reinterpret_cast<float*>(c->stage);
+    float* const dW = reinterpret_cast<float*>(c->d_stage);
     cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-    cudaMemsetAsync(gd->dLoss, 0, sizeof(float), c->stream);      // training steps leave theirs
+    cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);      // training steps leave theirs
     st = run_gradients(gd, gd->scratch, n);
     if (st != LF_OK) return st;
-    guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(gd->wGrad, gd->gGrad, gd->dLoss,
-                                                                                      1.f / (float)n, out);
-    cudaMemcpyAsync(dweights, out, kWeights * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(dgrid, out + kWeights, (size_t)kGridParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaMemcpyAsync(loss, out + kWeights + kGridParams, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(
+        gd->wGrad, gd->gGrad, gd->dLoss, 1.f / (float)n, dW, outGrid, dW + kWeights);
+    cudaMemcpyAsync(dgrid, outGrid, (size_t)kGridParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide gradients");
+    std::memcpy(dweights, hW, kWeights * sizeof(float));
+    *loss = hW[kWeights];
     return check_device(c);
 }
 
@@ -752,14 +758,15 @@ lf_status lf_guide_train(lf_guide* gd, const float* samples, int32_t n, float lr
     lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats);
     if (st != LF_OK) return st;
     cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-    cudaMemsetAsync(gd->dLoss, 0, sizeof(float), c->stream);
+    cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);
     st = lf_guide_train_device(gd, gd->scratch, n, lr);
     if (st != LF_OK) return st;
     if (loss)
     {
-        cudaMemcpyAsync(loss, gd->dLoss, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+        double sum = 0.0;
+        cudaMemcpyAsync(&sum, gd->dLoss, sizeof sum, cudaMemcpyDeviceToHost, c->stream);
         cudaStreamSynchronize(c->stream);
-        *loss /= (float)n;
+        *loss = (float)(sum / (double)n);
     }
     return check_device(c);
 }

@@ -287,7 +287,7 @@ int launch_infer_tc(const Net& net, const float* queries, const int* nDev, int c
                     cudaStream_t st);
 // One training pass on tcgen05 (lf_guide_tc.cu): the per-sample weight and grid gradients of n
 // sample records summed into gW / gGrid and the loss into `loss`, as the warp-level kernel.
-int launch_train_tc(const Net& net, const float* samples, int n, float* gW, float* gGrid, float* loss, uint32_t* status,
+int launch_train_tc(const Net& net, const float* samples, int n, float* gW, float* gGrid, double* loss, uint32_t* status,
                     cudaStream_t st);
 
 // Samples a direction from the compact mixture with uniforms u0 (lobe), u1, u2.

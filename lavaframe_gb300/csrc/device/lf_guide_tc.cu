@@ -18,11 +18,12 @@
 //
 // Training (guide_train_tc_kernel) runs the same forward pass with every activation tile kept
 // in shared memory, then the backward pass layer by layer: the output gradient dY (one row per
-// sample, FP16) times W^T gives the previous layer's gradient (M = 128 samples, K = out), and
+// sample, FP16) times W gives the previous layer's gradient (M = 128 samples, K = out), and
 // the weight gradient dW[out][in] += dY^T H sums over the tile's 128 samples as the MMA's K
 // dimension. For that product the row-per-sample tiles dY [s][out] and H [s][in] are read
 // MN-major (the transpose bits of the instruction descriptor): their 16-byte chunks run along
-// out and in, which for dW are the M and N dimensions. dY is kept 128 columns wide with zeros
+// out and in, which for dW are the M and N dimensions. The weights [out][in] are the dY product's B
+// operand MN-major in the same way, so one copy of them serves both passes. dY is kept 128 columns wide with zeros
 // beyond the layer's outputs, so dW is a 128-row MMA whose rows 0..63 are the layer's. The
 // four dW accumulators stay in TMEM across every tile the CTA processes and are added to the
 // global gradient once at the end; the grid-feature gradients are scattered with the
@@ -45,7 +46,7 @@ namespace guide
 namespace
 {
 constexpr int kTcRows = 128;                         // queries per tile = MMA M
-constexpr int kTcThreads = 128;                      // one thread per query (training)
+constexpr int kTrainThreads = 256;                   // training: two threads per sample
 constexpr int kTileBytes = kTcRows * kIn * 2;        // A tile: 128 x 64 FP16
 constexpr int kLayerBytes = 64 * 64 * 2;             // W1..W3: 64 x 64 FP16
 constexpr int kWBytes = 3 * kLayerBytes + kOut * 64 * 2;
@@ -169,56 +170,9 @@ __device__ __forceinline__ void load8(const unsigned char* tile, int row, int k0
     }
 }
 
-// The query's 64 input features (same values and FP16 rounding as encode_tile in lf_guide.cu)
-// into its row of the A tile.
-__device__ __forceinline__ void encode_row(const Net& net, const float* rec, bool valid, unsigned char* tile, int row)
-{
-    float f[64];
-    if (!valid)
-    {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) f[i] = 0.f;
-    }
-    else
-    {
-        float p01[3];
-        position01(net, rec, p01);
-#pragma unroll 1
-        for (int l = 0; l < kLevels; ++l)
-        {
-            float acc[4];
-            level_features(net, l, p01, acc);
-            // unrolled stores keep f[] in registers
-#pragma unroll
-            for (int q = 0; q < kLevels; ++q)
-                if (q == l)
-                {
-                    f[4 * q + 0] = acc[0];
-                    f[4 * q + 1] = acc[1];
-                    f[4 * q + 2] = acc[2];
-                    f[4 * q + 3] = acc[3];
-                }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-        {
-            const float* d = rec + 3 + 3 * h;   // outgoing direction, then the normal
-            float th, ph;
-            sph01(d[0], d[1], d[2], &th, &ph);
-#pragma unroll
-            for (int k = 0; k < kBlobBins; ++k)
-            {
-                f[32 + h * 16 + k] = blob(th, k);
-                f[32 + h * 16 + 8 + k] = blob(ph, k);
-            }
-        }
-    }
-#pragma unroll
-    for (int k0 = 0; k0 < 64; k0 += 8) store8(tile, row, k0, f + k0);
-}
-
-// Inference form of encode_row: the same FP16 values, written level by level (8 bytes at a
-// time) so that no 64-feature array stays live.
+// The query's 64 input features (same values and FP16 rounding as encode_tile in lf_guide.cu) into
+// its row of the A tile, written level by level (8 bytes at a time) so that no 64-feature array
+// stays live.
 __device__ __forceinline__ void encode_row_direct(const Net& net, const float* rec, bool valid, unsigned char* tile,
                                                   int row)
 {
@@ -437,20 +391,59 @@ namespace
 {
 // Shared memory of the training kernel, in this order so that every operand's span lies well
 // inside the allocation: dY (128 samples x 128 outputs, columns beyond the layer's outputs
-// zero), the input tile X and the activation tiles H1..H3 (128 x 64 each), the weights as
-// forward B operands [out][in] and as backward B operands W^T [in][out], then the mbarrier and
-// the TMEM address.
+// zero), the input tile X and the activation tiles H1..H3 (128 x 64 each), the weights
+// [out][in] (B operands of both passes), then the mbarrier and the TMEM address.
 constexpr int kDyBytes = 128 * 128 * 2;
 constexpr int kOffDy = 0;
 constexpr int kOffX = kOffDy + kDyBytes;
 constexpr int kOffH = kOffX + kTileBytes;                 // H1, H2, H3
 constexpr int kOffW = kOffH + 3 * kTileBytes;
-constexpr int kOffWT = kOffW + kWBytes;
-constexpr int kOffBar = kOffWT + kWBytes;
+constexpr int kOffBar = kOffW + kWBytes;
 constexpr int kTrainSmem = kOffBar + 16;
 constexpr uint32_t kTrainTmemCols = 512;                  // 2 x 64 forward/backward + 4 x 64 dW
 constexpr uint32_t kColDW = 128;                          // dW of layer l at kColDW + 64 l
 constexpr int kDyKg = 16;                                 // dY: 16 core matrices along its 128 columns
+
+// Adds four consecutive floats in one reduction (16-byte aligned).
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d)
+{
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+// Half h of a training sample's input row: levels 4 h .. 4 h + 3 and the one-blob bins of the outgoing
+// direction (h = 0) or the normal - the same FP16 values as encode_row_direct.
+__device__ __forceinline__ void encode_half(const Net& net, const float* rec, bool valid, int h, unsigned char* tile,
+                                            int row)
+{
+    if (!valid)
+    {
+#pragma unroll
+        for (int k0 = 0; k0 < 16; k0 += 8)
+        {
+            *reinterpret_cast<uint4*>(tile + cm_offset(row, 16 * h + k0)) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(tile + cm_offset(row, 32 + 16 * h + k0)) = make_uint4(0, 0, 0, 0);
+        }
+        return;
+    }
+    float p01[3];
+    position01(net, rec, p01);
+    float f[16];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) level_features(net, 4 * h + l, p01, f + 4 * l);
+    store8(tile, row, 16 * h, f);
+    store8(tile, row, 16 * h + 8, f + 8);
+    const float* d = rec + 3 + 3 * h;
+    float th, ph;
+    sph01(d[0], d[1], d[2], &th, &ph);
+#pragma unroll
+    for (int k = 0; k < kBlobBins; ++k)
+    {
+        f[k] = blob(th, k);
+        f[8 + k] = blob(ph, k);
+    }
+    store8(tile, row, 32 + 16 * h, f);
+    store8(tile, row, 32 + 16 * h + 8, f + 8);
+}
 
 // Issues one MMA group (k steps of K = 16) and commits it to the mbarrier; thread 0 only.
 __device__ __forceinline__ void issue(uint32_t dtmem, uint32_t a, uint32_t aStep, uint32_t aLbo, uint32_t aSbo, uint32_t b,
@@ -464,9 +457,14 @@ __device__ __forceinline__ void issue(uint32_t dtmem, uint32_t a, uint32_t aStep
 
 // One pass over n training samples: adds the per-sample gradients (not divided by n) of every
 // weight into gW and of every grid parameter into gGrid, and the summed loss into loss - the
-// same sums as guide_train_kernel, with the products on tcgen05.
-__global__ void __launch_bounds__(kTcThreads, 1)
-    guide_train_tc_kernel(Net net, const float* samples, int n, float* gW, float* gGrid, float* loss,
+// same sums as guide_train_kernel, with the products on tcgen05. Two threads per sample (threads
+// t and t + 128 have row t): each encodes and scatters half of the levels and takes half of
+// every accumulator's columns; the loss is the first one's. A tile is a chain of short steps, so a batch of
+// 16,384 (one tile per CTA) is bound by their latency and, before, by the reductions: of 70 us a
+// CTA spent 24 on 256 scalar reductions per sample, 24 on its weight gradients, 7 encoding, 7 on two
+// copies of the weights. 16,384 samples 89 -> 35 us.
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    guide_train_tc_kernel(Net net, const float* samples, int n, float* gW, float* gGrid, double* loss,
                           uint32_t* status)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -474,24 +472,21 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     unsigned char* sX = smem + kOffX;
     unsigned char* sH = smem + kOffH;
     unsigned char* sW = smem + kOffW;
-    unsigned char* sWT = smem + kOffWT;
     uint64_t* mbarPtr = reinterpret_cast<uint64_t*>(smem + kOffBar);
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(smem + kOffBar + 8);
     const int tid = threadIdx.x, warp = tid >> 5;
+    const int row = tid & 127, half = tid >> 7;
     const uint32_t mbar = smem_addr(mbarPtr);
 
-    // weights: forward B operands [out][in] (K = in) and backward B operands [in][out]
-    // (K = out: 8 core matrices for W1..W3, 6 for W4)
-    for (int i = tid; i < kWeights; i += kTcThreads)
+    // weights [out][in] in core matrices, 8 values at a time
+    for (int i = tid; i < kWeights / 8; i += kTrainThreads)
     {
-        const int l = i < 3 * 4096 ? i >> 12 : 3;
-        const int o = (i - l * 4096) >> 6, k = (i - l * 4096) & 63;
-        const __half w = net.W[i];
-        *reinterpret_cast<__half*>(sW + l * kLayerBytes + cm_offset(o, k)) = w;
-        *reinterpret_cast<__half*>(sWT + l * kLayerBytes + cm_offset(k, o, l < 3 ? 8 : 6)) = w;
+        const int l = i < 3 * 512 ? i >> 9 : 3;
+        const int o = (i - l * 512) >> 3, k = ((i - l * 512) & 7) * 8;
+        *reinterpret_cast<uint4*>(sW + l * kLayerBytes + cm_offset(o, k)) = reinterpret_cast<const uint4*>(net.W)[i];
     }
     // dY columns 64..127 stay zero (the padding rows of the dW products)
-    for (int i = tid; i < kDyBytes / 16; i += kTcThreads) reinterpret_cast<uint4*>(sDy)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < kDyBytes / 16; i += kTrainThreads) reinterpret_cast<uint4*>(sDy)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 0)
     {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmemSlot)),
@@ -509,9 +504,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem = *tmemSlot;
-    const uint32_t lane0 = (uint32_t)(warp * 32) << 16;
-    const uint32_t aDy = smem_addr(sDy), aX = smem_addr(sX), aH = smem_addr(sH), aW = smem_addr(sW),
-                   aWT = smem_addr(sWT);
+    const uint32_t lane0 = (uint32_t)((warp & 3) * 32) << 16;   // warps w and w + 4 read the same lanes
+    const uint32_t aDy = smem_addr(sDy), aX = smem_addr(sX), aH = smem_addr(sH), aW = smem_addr(sW);
     uint32_t phase = 0;
     bool failed = false, any = false;
     float lossSum = 0.f;
@@ -543,50 +537,55 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int tiles = (n + kTcRows - 1) / kTcRows;
     for (int tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x)
     {
-        const int q = tile * kTcRows + tid;
+        const int q = tile * kTcRows + row;
         const bool valid = q < n;
-        const float* rec = samples + (size_t)(valid ? q : 0) * kSampleFloats;
-        encode_row(net, rec, valid, sX, tid);
+        float rec[16];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            *reinterpret_cast<float4*>(rec + 4 * k) =
+                reinterpret_cast<const float4*>(samples + (size_t)(valid ? q : 0) * kSampleFloats)[k];
+        encode_half(net, rec, valid, half, sX, row);
         // forward: H1..H3 = relu(A W^T) into their tiles, outputs into registers
-        float out[48];
         for (int layer = 0; layer < 4 && !failed; ++layer)
         {
             const uint32_t a = layer == 0 ? aX : aH + (layer - 1) * kTileBytes;
             const uint32_t dcol = (uint32_t)(layer & 1) * 64u;
             failed = !run([&] { issue(tmem + dcol, a, 256, kLbo, kSbo, aW + layer * kLayerBytes, 256, kLbo, kSbo,
                                       layer < 3 ? idFwd : idOut, 4, false); });
-            if (failed) break;
-            if (layer < 3)
+            if (failed || layer == 3) break;
+            unsigned char* h = sH + layer * kTileBytes;
+#pragma unroll
+            for (int c0 = 0; c0 < 32; c0 += 16)
             {
-                unsigned char* h = sH + layer * kTileBytes;
-#pragma unroll
-                for (int c = 0; c < 64; c += 16)
-                {
-                    float v[16];
-                    tmem_ld16(tmem + lane0 + dcol + c, v);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
-                    store8(h, tid, c, v);
-                    store8(h, tid, c + 8, v + 8);
-                }
-            }
-            else
-            {
-#pragma unroll
-                for (int c = 0; c < kOut; c += 16) tmem_ld16(tmem + lane0 + dcol + c, out + c);
+                const int c = 32 * half + c0;
+                float v[16];
+                tmem_ld16(tmem + lane0 + dcol + c, v);
                 tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+                store8(h, row, c, v);
+                store8(h, row, c + 8, v + 8);
             }
         }
         if (failed) break;
         // loss and the output gradient (40 used of 48; columns 40..63 zero)
+        if (half == 0)
         {
-            float d[64];
+            float out[48], d[40];
 #pragma unroll
-            for (int k = 0; k < 64; ++k) d[k] = 0.f;
+            for (int c = 0; c < kOut; c += 16) tmem_ld16(tmem + lane0 + 64u + c, out + c);
+            tmem_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 40; ++k) d[k] = 0.f;
             if (valid) lossSum += sample_loss_grad(out, rec + 9, rec[12], d);
 #pragma unroll
-            for (int k0 = 0; k0 < 64; k0 += 8) store8(sDy, tid, k0, d + k0, kDyKg);
+            for (int k0 = 0; k0 < 40; k0 += 8) store8(sDy, row, k0, d + k0, kDyKg);
+        }
+        else
+        {
+#pragma unroll
+            for (int k0 = 40; k0 < 64; k0 += 8)
+                *reinterpret_cast<uint4*>(sDy + cm_offset(row, k0, kDyKg)) = make_uint4(0, 0, 0, 0);
         }
         // backward, layer 4 .. 1: dH = dY W (into the free forward column half) and
         // dW += dY^T H (accumulated across tiles); then dY of the layer below = dH * relu'(H)
@@ -598,9 +597,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const int nIn = layer == 0 ? 32 : 64;                                    // input gradients needed
             const bool accW = any;
             failed = !run([&] {
-                // dH[s][in] = sum_out dY[s][out] W[out][in]: A = dY (K-major, K = out), B = W^T
-                issue(tmem + dcol, aDy, 256, kLbo, kDyKg * 128, aWT + layer * kLayerBytes, 256, kLbo,
-                      (layer < 3 ? 8 : 6) * 128, instr_desc(kTcRows, nIn), kSteps, false);
+                // dH[s][in] = sum_out dY[s][out] W[out][in]: A = dY (K-major, K = out), B = W read
+                // MN-major (N = inputs, K = its rows)
+                issue(tmem + dcol, aDy, 256, kLbo, kDyKg * 128, aW + layer * kLayerBytes, 2 * 1024, 1024, 128,
+                      instr_desc(kTcRows, nIn, false, true), kSteps, false);
                 // dW[out][in] += sum_s dY[s][out] H[s][in]: A = dY^T (MN-major, M = 128 padded
                 // outputs), B = H^T (MN-major, N = 64 inputs); K = the tile's 128 samples
                 issue(tmem + kColDW + 64 * layer, aDy, 2 * kDyKg * 128, kDyKg * 128, 128, hIn, 2 * 1024, 1024, 128,
@@ -612,75 +612,73 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 // dY of layer - 1 = dH masked by the ReLU of H_layer (its FP16 activations > 0)
                 const unsigned char* h = sH + (layer - 1) * kTileBytes;
 #pragma unroll
-                for (int c = 0; c < 64; c += 16)
+                for (int c0 = 0; c0 < 32; c0 += 16)
                 {
+                    const int c = 32 * half + c0;
                     float v[16], hv[16];
                     tmem_ld16(tmem + lane0 + dcol + c, v);
                     tmem_wait_ld();
-                    load8(h, tid, c, hv);
-                    load8(h, tid, c + 8, hv + 8);
+                    load8(h, row, c, hv);
+                    load8(h, row, c + 8, hv + 8);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) v[i] = hv[i] > 0.f ? v[i] : 0.f;
-                    store8(sDy, tid, c, v, kDyKg);
-                    store8(sDy, tid, c + 8, v + 8, kDyKg);
+                    store8(sDy, row, c, v, kDyKg);
+                    store8(sDy, row, c + 8, v + 8, kDyKg);
                 }
             }
             else
             {
-                // grid-feature gradients (inputs 0..31) scattered with the trilinear weights; the
-                // warp-wide TMEM loads run on every lane, the scatter on valid samples only
-                float dx[32];
-#pragma unroll
-                for (int c = 0; c < 32; c += 16) tmem_ld16(tmem + lane0 + dcol + c, dx + c);
+                // grid-feature gradients (inputs 0..31) scattered with the trilinear weights, four
+                // features per reduction; the warp-wide TMEM loads run on every lane, the scatter on
+                // valid samples only
+                float dx[16];
+                tmem_ld16(tmem + lane0 + dcol + 16 * half, dx);
                 tmem_wait_ld();
                 float p01[3];
                 position01(net, rec, p01);
-#pragma unroll 1
-                for (int l = 0; l < (valid ? kLevels : 0); ++l)
+                if (valid)
                 {
-                    uint32_t idx[8];
-                    float w[8];
-                    grid_corners(net.res[l], p01, idx, w);
-                    float* gt = gGrid + (size_t)l * kT * kFeatures;
-                    float g4[4];
 #pragma unroll
-                    for (int f = 0; f < 4; ++f)
+                    for (int j = 0; j < 4; ++j)
                     {
-                        g4[f] = dx[0];
+                        const int l = 4 * half + j;
+                        uint32_t idx[8];
+                        float w[8];
+                        grid_corners(net.res[l], p01, idx, w);
+                        float* gt = gGrid + (size_t)l * kT * kFeatures;
 #pragma unroll
-                        for (int qq = 0; qq < 32; ++qq)
-                            if (qq == l * 4 + f) g4[f] = dx[qq];
+                        for (int c = 0; c < 8; ++c)
+                            red_add4(gt + (size_t)idx[c] * kFeatures, w[c] * dx[4 * j], w[c] * dx[4 * j + 1],
+                                     w[c] * dx[4 * j + 2], w[c] * dx[4 * j + 3]);
                     }
-                    for (int c = 0; c < 8; ++c)
-                        for (int f = 0; f < 4; ++f) atomicAdd(&gt[(size_t)idx[c] * kFeatures + f], w[c] * g4[f]);
                 }
             }
         }
         any = true;
     }
-    // loss: block sum, one atomic
+    // loss: warp sums, added in double so that the sum's rounding does not grow with the batch
     for (int off = 16; off > 0; off >>= 1) lossSum += __shfl_xor_sync(0xffffffffu, lossSum, off);
-    if ((tid & 31) == 0 && lossSum != 0.f) atomicAdd(loss, lossSum);
-    // weight gradients: TMEM lanes 0..63 = outputs, 64 columns = inputs, one atomic each
+    if ((tid & 31) == 0 && lossSum != 0.f) atomicAdd(loss, (double)lossSum);
+    // weight gradients: TMEM lanes 0..63 = outputs, 64 columns = inputs, four per reduction. Warps 0 and
+    // 4 hold lanes 0..31, warps 1 and 5 lanes 32..63; each takes half of the columns, and the CTAs
+    // start at different layers, so that they do not all add to the same lines at a time.
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    if (!failed && any && warp < 2)
+    if (!failed && any && (warp & 3) < 2)
     {
-        for (int layer = 0; layer < 4; ++layer)
+        const int o = row;   // lanes 0..63
+        for (int k = 0; k < 8; ++k)
         {
-            const int o = tid;   // lanes 0..63: warps 0 and 1
+            const int part = (k + blockIdx.x) & 7, layer = part >> 1, c = 32 * half + 16 * (part & 1);
             const int outs = layer < 3 ? 64 : kOut;
-            const int base = layer * 4096;
-            for (int c = 0; c < 64; c += 16)
-            {
-                float v[16];
-                tmem_ld16(tmem + lane0 + kColDW + 64 * layer + c, v);
-                tmem_wait_ld();
-                if (o < outs)
-                    for (int i = 0; i < 16; ++i)
-                        if (v[i] != 0.f) atomicAdd(&gW[base + o * 64 + c + i], v[i]);
-            }
+            float v[16];
+            tmem_ld16(tmem + lane0 + kColDW + 64 * layer + c, v);
+            tmem_wait_ld();
+            if (o < outs)
+#pragma unroll
+                for (int i = 0; i < 16; i += 4)
+                    red_add4(&gW[layer * 4096 + o * 64 + c + i], v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
     }
     fence_before_sync();
@@ -693,7 +691,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
 }
 
-int launch_train_tc(const Net& net, const float* samples, int n, float* gW, float* gGrid, float* loss, uint32_t* status,
+int launch_train_tc(const Net& net, const float* samples, int n, float* gW, float* gGrid, double* loss, uint32_t* status,
                     cudaStream_t st)
 {
     static bool attr = false;
@@ -708,7 +706,7 @@ int launch_train_tc(const Net& net, const float* samples, int n, float* gW, floa
     // one CTA per SM: its 512 TMEM columns are the SM's
     const int tiles = (n + kTcRows - 1) / kTcRows;
     const int blocks = std::max(1, std::min(sms, tiles));
-    guide_train_tc_kernel<<<blocks, kTcThreads, kTrainSmem, st>>>(net, samples, n, gW, gGrid, loss, status);
+    guide_train_tc_kernel<<<blocks, kTrainThreads, kTrainSmem, st>>>(net, samples, n, gW, gGrid, loss, status);
     return (int)cudaGetLastError();
 }
 

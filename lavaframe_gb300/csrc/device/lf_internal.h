@@ -63,7 +63,7 @@ struct lf_ctx
     size_t binCap = 0;
     uint32_t* binHist = nullptr;
     unsigned long long* binNext = nullptr;   // fetch counter and blocks done, zero between launches
-    char* stage = nullptr;                   // page-locked staging of small host queries
+    char* stage = nullptr;                   // page-locked staging block (ensure_stage)
     char* d_stage = nullptr;                 // its device address
     lfrt::EngineHost* engine = nullptr;   // multi-job engine, created on first use
     // traversal-kernel timer of the binned ray queries: one event pair per launch while on
@@ -187,6 +187,10 @@ inline lf_status check_device(lf_ctx* c)
 // whole frame unless the parameters set a tile size.
 void fill_params(Params& P, const lf_render_params* p, const lf_scene* sc);
 
+// Page-locked staging of small results and queries, mapped for the kernels (c->stage, c->d_stage);
+// false when there is none.
+constexpr size_t kStageBytes = size_t(1) << 18;
+bool ensure_stage(lf_ctx* c);
 // The copy streams and events of calls that overlap copies with kernels, made on first use.
 cudaError_t ensure_chunk_streams(lf_ctx* c);
 // The colour channels of n padded pixels into host memory, after the stream's work (synchronises).

@@ -1004,6 +1004,21 @@ size_t lf_scene_device_bytes(const lf_scene* sc) { return sc ? sc->bytes : 0; }
 
 namespace lfrt
 {
+// The context's page-locked staging block, mapped for the kernels; false when there is none.
+bool ensure_stage(lf_ctx* c)
+{
+    if (c->stage) return true;
+    if (cudaHostAlloc((void**)&c->stage, kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&c->d_stage, c->stage, 0) != cudaSuccess)
+    {
+        cudaGetLastError();
+        if (c->stage) cudaFreeHost(c->stage);
+        c->stage = nullptr;
+        return false;
+    }
+    return true;
+}
+
 cudaError_t ensure_chunk_streams(lf_ctx* c)
 {
     if (c->copyOut) return cudaSuccess;
@@ -1152,23 +1167,6 @@ char* mapped_range(const lf_ctx* c, const void* p, size_t bytes)
         if (h.dev && q >= h.host && bytes <= h.bytes && (size_t)(q - h.host) <= h.bytes - bytes)
             return h.dev + (q - h.host);
     return nullptr;
-}
-
-constexpr size_t kStageBytes = size_t(1) << 18;
-
-// The context's page-locked staging block, mapped for the kernels; false when there is none.
-bool ensure_stage(lf_ctx* c)
-{
-    if (c->stage) return true;
-    if (cudaHostAlloc((void**)&c->stage, kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&c->d_stage, c->stage, 0) != cudaSuccess)
-    {
-        cudaGetLastError();
-        if (c->stage) cudaFreeHost(c->stage);
-        c->stage = nullptr;
-        return false;
-    }
-    return true;
 }
 
 void read_trace_stats(lf_ctx* c)
