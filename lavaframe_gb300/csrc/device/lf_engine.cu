@@ -144,6 +144,49 @@ __device__ __forceinline__ bool last_block(int* counter)
     }
     return last;   // of thread 0; false elsewhere
 }
+
+// QueueShare for blocks that keep together: the warps of a block take neighbouring chunks, and the
+// block takes its next ones from the counter at once. Every thread of the block calls next().
+struct BlockShare
+{
+    int n, chunk, base;   // base: the warp's chunk; may lie beyond n while other warps' do not
+    int block;            // the block's first entry
+
+    __device__ __forceinline__ explicit BlockShare(int entries) : n(entries)
+    {
+        const int nw = blockDim.x >> 5;
+        const int warps = nw * gridDim.x;
+        chunk = n < 32 * warps ? (n + warps - 1) / warps : 32;
+        take((long long)blockIdx.x * nw * chunk);
+    }
+    __device__ __forceinline__ void take(long long first)
+    {
+        block = first < n ? (int)first : n;
+        const long long b = (long long)block + (int)(threadIdx.x >> 5) * chunk;
+        base = b < n ? (int)b : n;
+    }
+    __device__ __forceinline__ bool more() const { return block < n; }
+    __device__ __forceinline__ int entry() const
+    {
+        const int lane = threadIdx.x & 31;
+        return lane < chunk && lane < n - base ? base + lane : -1;
+    }
+    __device__ __forceinline__ void next(int* counter)
+    {
+        const int nw = blockDim.x >> 5;
+        const long long once = (long long)gridDim.x * nw * chunk;
+        if (n <= once)
+        {
+            block = n;
+            return;
+        }
+        __shared__ int got;
+        __syncthreads();
+        if (threadIdx.x == 0) got = atomicAdd(counter, nw * chunk);
+        __syncthreads();
+        take(got < n - once ? once + got : (long long)n);
+    }
+};
 }
 
 // ------------------------------------------------------------------ init / append
@@ -616,61 +659,73 @@ __global__ void __maxnreg__(64) engine_shadow_kernel(EngineBuffers b, EngineJob 
 }
 
 // ------------------------------------------------------------------ drain
-// The last paths of a run, once no ids are left to issue: every queued path is taken through
-// its remaining bounces by one thread (extension, shade, next-event rays, in the order of the
-// step kernels) and written out. Per path this is the same sequence of operations the step
-// kernels perform, so results and ray counts are unchanged; what goes away is one launch
-// sequence per bounce whose length is set by the slowest ray of an almost empty pool.
-// One path from its queued extension ray to its end; returns the extension and shadow rays
-// it traced.
-template <bool kLights = true>
-__device__ __forceinline__ void run_path(const ShadeScene& S, const Params& P, const PathSoA& ps, uint32_t* status,
-                                         unsigned long long* ctr, int p, unsigned long long& ext,
-                                         unsigned long long& shadowRays)
+// Paths run to their ends by one thread each: the operations of the step kernels in their order, so
+// results and ray counts are unchanged; what goes away is one launch sequence per bounce whose length
+// is set by the slowest ray of an almost empty pool.
+//
+// The block's threads go through a bounce's three parts together. Traversal, shading and occlusion in
+// one kernel are more code than the instruction caches hold, and warps that drift apart fetch all of
+// it all the time (15 of 24 stall cycles per issue with 128-thread blocks and no barriers); in step they
+// share what they fetch. Without / with barriers, us: 62k paths of the Cornell box 193 / 118, a room 531 /
+// 349, random triangles 510 / 531, spheres 447 / 521; 131k paths 369 / 203, 923 / 581, 688 / 833,
+// 626 / 600. Blocks of 128 threads wait less and share less (138, 388, 530, 513 at 62k), of 512 and
+// 640 the other way.
+constexpr int kRunBlock = 256;
+
+// Takes the path in slot p (-1: none) of every thread of the block from its extension ray to its end;
+// adds up the extension and shadow rays. `job()` gives the scene and parameters of the thread's path.
+template <bool kLights, class Job>
+__device__ __forceinline__ void run_paths(const PathSoA& ps, uint32_t* status, unsigned long long* ctr, int p, Job job,
+                                          unsigned long long& ext, unsigned long long& shadowRays)
 {
-    for (int bounce = 0; bounce < 4096; ++bounce)
+    bool alive = p >= 0;
+    for (int bounce = 0; bounce < 4096 && __syncthreads_or(alive); ++bounce)
     {
-        const float4 o4 = ps.o[p], d4 = ps.d[p];
-        Hit h;
-        const uint32_t err = closest_hit<false>(S.trav, f3(o4), f3(d4), kInfinity, P.useLights != 0, &h, nullptr);
-        ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));
-        set_error(status, err);
-        ++ext;
+        if (alive)
+        {
+            const EngineJob& J = job();
+            const float4 o4 = ps.o[p], d4 = ps.d[p];
+            Hit h;
+            const uint32_t err = closest_hit<false>(J.S.trav, f3(o4), f3(d4), kInfinity, J.P.useLights != 0, &h, nullptr);
+            ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));
+            set_error(status, err);
+            ++ext;
+        }
+        __syncthreads();
         bool pushExt = false, pushShadow = false;
         ShadowRec rec;
-        shade_path<kLights>(S, P, ps, p, ctr, pushExt, pushShadow, rec);
-        if (pushShadow) set_error(status, shadow_path(S, P, ps, &rec, shadowRays));
-        if (!pushExt) return;
+        if (alive) shade_path<kLights>(job().S, job().P, ps, p, ctr, pushExt, pushShadow, rec);
+        __syncthreads();
+        if (pushShadow) set_error(status, shadow_path(job().S, job().P, ps, &rec, shadowRays));
+        alive = pushExt;
     }
 }
 
-// More than `limit` queued paths are left for the step kernels.
+// The last paths of a run, once no ids are left to issue: every queued path to its end. More than
+// `limit` queued paths are left for the step kernels.
 template <bool kOne>
-__global__ void __launch_bounds__(128) engine_drain_kernel(EngineBuffers b, EngineJob one, int parity, int limit)
+__global__ void __launch_bounds__(kRunBlock) engine_drain_kernel(EngineBuffers b, EngineJob one, int parity, int limit)
 {
-    if (b.ctl->count[parity] > limit || b.ctl->count[parity] == 0) return;
+    const int n = b.ctl->count[parity];
+    if (n > limit || n == 0) return;
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
     EngineCtl* ctl = b.ctl;
-    const int n = ctl->count[parity];
     const int* q = b.queue[parity];
     unsigned long long ext = 0, shadowRays = 0;
-    for (QueueShare share(n); share.more(); share.next(&ctl->extendNext))
+    for (BlockShare share(n); share.more(); share.next(&ctl->extendNext))
     {
         const int i = share.entry();
-        if (i >= 0)
+        const int p = i >= 0 ? q[i] : -1;
+        if constexpr (kOne)
+            run_paths<true>(b.ps, b.status, b.ctr, p, [&]() -> const EngineJob& { return one; }, ext, shadowRays);
+        else
         {
-            const int p = q[i];
-            if constexpr (kOne)
-                run_path(one.S, one.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
-            else
-            {
-                const EngineJob& J = b.jobs[job_of(reinterpret_cast<const int*>(b.ps.info)[4 * p + 3])];
-                run_path(J.S, J.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
-            }
-            end_path(b, p, b.ps.info[p], b.ps.L[p], td, bd);
+            const EngineJob* J = p >= 0 ? b.jobs + job_of(reinterpret_cast<const int*>(b.ps.info)[4 * p + 3]) : b.jobs;
+            run_paths<true>(b.ps, b.status, b.ctr, p, [&]() -> const EngineJob& { return *J; }, ext, shadowRays);
         }
+        if (p >= 0) end_path(b, p, b.ps.info[p], b.ps.L[p], td, bd);
     }
     warp_count_add(&b.ctr[1], ext);
     warp_count_add(&b.ctr[2], shadowRays);
@@ -729,25 +784,23 @@ __global__ void __launch_bounds__(256) engine_start_kernel(EngineBuffers b, Para
 }
 
 // A whole small run in one launch: every thread takes paths from their camera ray to their end
-// (the operations of the step kernels in their order, so results and ray counts are unchanged),
-// without queues. b.ps.L is the run's radiance array: a path's slot is its radiance entry, so an
-// ended path needs no write-out, and the slots stay marked free (info.w = -1). kDirectPaths
-// says where it pays.
+// (run_paths), without queues. b.ps.L is the run's radiance array: a path's slot is its radiance
+// entry, so an ended path needs no write-out, and the slots stay marked free (info.w = -1).
+// kDirectPaths says where it pays.
 template <bool kLights>
-__global__ void __launch_bounds__(128) engine_direct_kernel(EngineBuffers b, EngineJob one, EnginePass first,
-                                                            const EnginePass* table, int numPasses, int n)
+__global__ void __launch_bounds__(kRunBlock) engine_direct_kernel(EngineBuffers b, EngineJob one, EnginePass first,
+                                                                  const EnginePass* table, int numPasses, int n)
 {
     unsigned long long ext = 0, shadowRays = 0;
-    for (QueueShare share(n); share.more(); share.next(&b.ctl->extendNext))
+    for (BlockShare share(n); share.more(); share.next(&b.ctl->extendNext))
     {
         const int i = share.entry();
+        int p = -1;
         if (i >= 0)
-        {
-            const int p = start_path(b.ps, one.P, first, table, numPasses, i, false,
-                                     [](const EnginePass& Q, int entry) { return (int)Q.pathBase + entry; });
-            if (one.P.maxDepth > 0) run_path<kLights>(one.S, one.P, b.ps, b.status, b.ctr, p, ext, shadowRays);
-        }
-        __syncwarp();
+            p = start_path(b.ps, one.P, first, table, numPasses, i, false,
+                           [](const EnginePass& Q, int entry) { return (int)Q.pathBase + entry; });
+        if (one.P.maxDepth > 0)
+            run_paths<kLights>(b.ps, b.status, b.ctr, p, [&]() -> const EngineJob& { return one; }, ext, shadowRays);
     }
     warp_count_add(&b.ctr[1], ext);
     warp_count_add(&b.ctr[2], shadowRays);
@@ -842,17 +895,16 @@ __global__ void engine_accumulate_run_kernel(int width, int height, int tileW, i
 // ------------------------------------------------------------------ launchers
 namespace
 {
-// Runs of up to kDirectPaths paths are traced by one launch. Kernel by kernel every bounce waits for
-// its slowest ray three times over; one thread per path overlaps those waits, but its code (traversal,
-// shading and occlusion in one kernel) overflows the instruction caches once the GPU is full (15 of
-// 24 stall cycles per issue at 262k paths). One launch / kernel by kernel, us: 4096 paths 113 / 166
-// (Cornell box), 266 / 386 (room), 214 / 400 (random triangles), 200 / 412 (spheres); 62k paths
-// 204 / 231, 549 / 587, 594 / 678, 477 / 771; 131k paths 388 / 254, 957 / 732, 776 / 917, 657 / 996.
-constexpr int kDirectPaths = 1 << 16;
+// Runs of up to kDirectPaths paths are traced by one launch: kernel by kernel every bounce waits for
+// the slowest ray of the whole run three times over, in one kernel only for the slowest of a block. One
+// launch / kernel by kernel, us: 4096 paths 85 / 166 (Cornell box), 197 / 386 (room), 247 / 400
+// (random triangles), 206 / 412 (spheres); 62k paths 117 / 231, 338 / 587, 505 / 678, 504 / 771; 131k paths
+// 202 / 254, 579 / 716, 837 / 826, 621 / 926; 205k paths 292 / 305, 824 / 766, 1283 / 1134, 753 / 971.
+constexpr int kDirectPaths = 1 << 17;
 // A run takes its paths to their ends in the drain after the second or fourth bounce once this many
-// are left: spheres 262k paths 1321 -> 1104 us, room 1M paths 2073 -> 2092; with 65,536 the room's
-// 2148, with 16,384 the spheres' 524k paths 1272 -> 1360.
-constexpr int kDrainPaths = 1 << 15;
+// are left: room 1M paths 2037 (half as many) -> 1980 us, spheres 1M 1642 -> 1542; twice as many cost the
+// random triangles' 262k paths 10 %.
+constexpr int kDrainPaths = 1 << 16;
 constexpr int kRunBounces = 16;   // bounces of a run in steps; deeper paths are taken to their ends by the drain
 
 int sm_count()
@@ -937,8 +989,8 @@ void step(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream_t
 template <bool kOne>
 void drain(const EngineBuffers& b, const EngineJob& one, int parity, int n, int limit, cudaStream_t st)
 {
-    engine_drain_kernel<kOne><<<full_grid((const void*)engine_drain_kernel<kOne>, 128, (long long)n * 32), 128, 0, st>>>(
-        b, one, parity, limit);
+    engine_drain_kernel<kOne><<<full_grid((const void*)engine_drain_kernel<kOne>, kRunBlock, (long long)n * 32), kRunBlock, 0,
+                                st>>>(b, one, parity, limit);
 }
 
 template <bool kOne>
@@ -961,8 +1013,8 @@ int launch_frame_run(const EngineBuffers& b0, const EngineJob& one, const Engine
     {
         b.ps.L = radiance;
         auto direct = [&](auto kernel) {
-            kernel<<<full_grid((const void*)kernel, 128, (long long)n * 32), 128, 0, st>>>(b, one, first, table, numPasses,
-                                                                                          n);
+            kernel<<<full_grid((const void*)kernel, kRunBlock, (long long)n * 32), kRunBlock, 0, st>>>(b, one, first, table,
+                                                                                                      numPasses, n);
         };
         one.P.useLights ? direct(engine_direct_kernel<true>) : direct(engine_direct_kernel<false>);
         return (int)cudaGetLastError();

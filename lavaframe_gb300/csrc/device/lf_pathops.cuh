@@ -78,17 +78,17 @@ __device__ __forceinline__ void warp_count_add(unsigned long long* counter, unsi
 // A kernel's share of n queue entries: warps take `chunk` entries at a time, the first chunk by
 // their place in the grid and further ones from a counter, so that long rays do not hold up a
 // fixed share and a queue of one chunk per warp needs no atomics (8,500 of them on one address
-// cost about 8 us). The chunk is 32, or fewer (a power of two) while the entries do not give every
-// warp of the grid a chunk: a thin queue is a chain of dependent loads per path, and a warp runs
+// cost about 8 us). The chunk is 32, or fewer while the entries do not give every warp of the grid a
+// chunk: a thin queue is a chain of dependent loads per path, and a warp runs
 // the union of its lanes' branches (20,000 paths on spheres 1189 -> 755 us, in a room 667 -> 486).
 struct QueueShare
 {
     int n, chunk, base;
 
-    __device__ __forceinline__ explicit QueueShare(int entries) : n(entries), chunk(32)
+    __device__ __forceinline__ explicit QueueShare(int entries) : n(entries)
     {
         const int warps = gridDim.x * (blockDim.x >> 5);
-        while (chunk > 1 && (long long)(chunk >> 1) * warps >= n) chunk >>= 1;
+        chunk = n < 32 * warps ? (n + warps - 1) / warps : 32;
         const long long first = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk;
         base = first < n ? (int)first : n;
     }

@@ -30,13 +30,15 @@ SCENES = {"cornell": lambda: lf.HostScene().gen_cornell(64, 64), "spheres": lamb
 @pytest.mark.parametrize("size,spp,depth,tile,batch,flags", [
     ((1, 1), 1, 4, 0, 0, 0),
     ((33, 7), 3, 3, 0, 2, 0),          # one launch over two passes
-    ((256, 256), 1, 4, 0, 0, 0),       # the largest one-launch run
-    ((257, 256), 1, 4, 0, 0, 0),       # the smallest run in steps
+    ((251, 67), 2, 5, 0, 0, 0),        # one launch, chunks that do not divide
+    ((512, 256), 1, 4, 0, 0, 0),       # the largest one-launch run
+    ((513, 256), 1, 4, 0, 0, 0),       # the smallest run in steps
     ((300, 120), 4, 1, 0, 0, 0),       # a single bounce
     ((300, 120), 4, 20, 0, 0, 0),      # deeper than the bounces in steps
-    ((300, 120), 4, 5, 0, 3, 0),       # passes in steps
-    ((300, 120), 4, 6, (64, 50), 2, 0),
-    ((300, 120), 4, 6, (64, 50), 2, lf.FRAME_TILED_FRAMES),
+    ((300, 120), 5, 20, 0, 0, 0),
+    ((300, 120), 5, 5, 0, 3, 0),       # passes in steps
+    ((300, 120), 5, 6, (64, 50), 2, 0),
+    ((300, 120), 5, 6, (64, 50), 2, lf.FRAME_TILED_FRAMES),
     ((90, 60), 2, 6, (32, 32), 0, lf.FRAME_TILED_FRAMES),
     ((90, 60), 2, 0, (32, 32), 0, 0),  # depth 0
 ])
