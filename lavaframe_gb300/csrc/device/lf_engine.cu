@@ -118,6 +118,17 @@ __device__ __forceinline__ unsigned long long find_pass(const EnginePass* passes
 namespace
 {
 
+// The kernels of a run form a chain in which each needs all of the one before: launched with
+// programmatic serialization (launch_chained), a kernel's blocks take the places that the blocks of the
+// one before leave and wait here for the rest of it, so that neither the launch nor the end of a
+// kernel leaves the GPU idle. Every kernel of a chain calls this first; launched otherwise it does nothing.
+// 262k paths: Cornell box 352 -> 324 us, room 876 -> 820, spheres 996 -> 947; 1M paths 1-4 %.
+__device__ __forceinline__ void chain_kernels()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Clears the work counters of a step.
 __device__ __forceinline__ void reset_step(EngineCtl* c)
 {
@@ -238,6 +249,7 @@ constexpr int kRefillGroups = 4;   // groups of kRefillBlock slots a refill bloc
 // slots. A thread loads four entries' state before it writes any.
 __global__ void __launch_bounds__(256) engine_finish_kernel(EngineBuffers b, int parity)
 {
+    chain_kernels();
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
@@ -296,6 +308,7 @@ __device__ __forceinline__ int warp_exclusive_scan(int& v)
 template <bool kOne>
 __global__ void __launch_bounds__(kRefillBlock) engine_refill_kernel(EngineBuffers b, EngineJob one, int parity)
 {
+    chain_kernels();
     constexpr int kG = kRefillGroups;
     constexpr int kW = kRefillBlock / 32;
     static_assert(kG * kW == 32, "one scan entry per lane of a warp");
@@ -461,6 +474,7 @@ __global__ void __launch_bounds__(kRefillBlock) engine_refill_kernel(EngineBuffe
 template <bool kOne>
 __global__ void __maxnreg__(72) engine_extend_kernel(EngineBuffers b, EngineJob one, int parity)
 {
+    chain_kernels();
     const int n = b.ctl->count[parity];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&b.ctr[1], (unsigned long long)n);
     const int* q = b.queue[parity];
@@ -545,6 +559,7 @@ template <bool kOne, int kThreadsPerSm, bool kLights = true>
 __global__ void __launch_bounds__(256, kThreadsPerSm ? kThreadsPerSm / 256 : 1)
     engine_shade_kernel(EngineBuffers b, EngineJob one, int parity)
 {
+    chain_kernels();
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
@@ -623,6 +638,7 @@ __global__ void __launch_bounds__(256, kThreadsPerSm ? kThreadsPerSm / 256 : 1)
 template <bool kOne>
 __global__ void __maxnreg__(64) engine_shadow_kernel(EngineBuffers b, EngineJob one, int parity)
 {
+    chain_kernels();
     __shared__ BlockDone bd;
     block_done_begin(bd);
     ThreadDone td;
@@ -706,6 +722,7 @@ __device__ __forceinline__ void run_paths(const PathSoA& ps, uint32_t* status, u
 template <bool kOne>
 __global__ void __launch_bounds__(kRunBlock) engine_drain_kernel(EngineBuffers b, EngineJob one, int parity, int limit)
 {
+    chain_kernels();
     const int n = b.ctl->count[parity];
     if (n > limit || n == 0) return;
     __shared__ BlockDone bd;
@@ -771,6 +788,7 @@ __device__ __forceinline__ int start_path(const PathSoA& ps, const Params& P, co
 __global__ void __launch_bounds__(256) engine_start_kernel(EngineBuffers b, Params P, EnginePass first, EnginePass* table,
                                                            int numPasses, int n)
 {
+    chain_kernels();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid == 0)
     {
@@ -791,6 +809,7 @@ template <bool kLights>
 __global__ void __launch_bounds__(kRunBlock) engine_direct_kernel(EngineBuffers b, EngineJob one, EnginePass first,
                                                                   const EnginePass* table, int numPasses, int n)
 {
+    chain_kernels();
     unsigned long long ext = 0, shadowRays = 0;
     for (BlockShare share(n); share.more(); share.next(&b.ctl->extendNext))
     {
@@ -810,6 +829,7 @@ __global__ void __launch_bounds__(kRunBlock) engine_direct_kernel(EngineBuffers 
 // ------------------------------------------------------------------ accumulate
 __global__ void engine_accumulate_kernel(int width, int tileW, int tileH, EnginePass Q, float4* accum, double* accum64)
 {
+    chain_kernels();
     const int visPix = Q.visW * Q.visH;
     for (int lp = blockIdx.x * blockDim.x + threadIdx.x; lp < visPix; lp += gridDim.x * blockDim.x)
     {
@@ -851,6 +871,7 @@ __global__ void engine_accumulate_kernel(int width, int tileW, int tileH, Engine
 __global__ void engine_accumulate_run_kernel(int width, int height, int tileW, int tileH, const EnginePass* table,
                                              int chunks, int tilesX, int tilesY, float4* accum, double* accum64)
 {
+    chain_kernels();
     for (int gpix = blockIdx.x * blockDim.x + threadIdx.x; gpix < width * height; gpix += gridDim.x * blockDim.x)
     {
         const int x = gpix % width, y = gpix / width;
@@ -920,6 +941,21 @@ int sm_count()
     return n;
 }
 
+template <class... Formal, class... Actual>
+void launch_chained(void (*kernel)(Formal...), int grid, int block, cudaStream_t st, const Actual&... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 int full_grid(const void* kernel, int block, long long work)
 {
     const int per_sm = occupancy_blocks_per_sm(kernel, block);
@@ -950,10 +986,10 @@ void refill(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream
 {
     const int BF = 256;
     if (!kOne || one.P.maxDepth <= 0)   // only depth-0 paths are on the done list
-        engine_finish_kernel<<<full_grid((const void*)engine_finish_kernel, BF, b.cap), BF, 0, st>>>(b, parity);
-    engine_refill_kernel<kOne><<<full_grid((const void*)engine_refill_kernel<kOne>, kRefillBlock,
-                                           (long long)b.cap / kRefillGroups),
-                                 kRefillBlock, 0, st>>>(b, one, parity);
+        launch_chained(engine_finish_kernel, full_grid((const void*)engine_finish_kernel, BF, b.cap), BF, st, b, parity);
+    launch_chained(engine_refill_kernel<kOne>,
+                   full_grid((const void*)engine_refill_kernel<kOne>, kRefillBlock, (long long)b.cap / kRefillGroups),
+                   kRefillBlock, st, b, one, parity);
 }
 
 // One bounce of the queued paths, at most n of them.
@@ -965,8 +1001,8 @@ void bounce(const EngineBuffers& b, const EngineJob& one, int parity, int n, cud
     const int bw = b.blockShadow > 0 ? b.blockShadow : 128;
     // grids for one path per warp at least: thin queues are spread over the GPU (QueueShare)
     auto grid = [&](const void* k, int block) { return full_grid(k, block, (long long)n * 32); };
-    auto shade = [&](auto kernel) { kernel<<<grid((const void*)kernel, bs), bs, 0, st>>>(b, one, parity); };
-    engine_extend_kernel<kOne><<<grid((const void*)engine_extend_kernel<kOne>, be), be, 0, st>>>(b, one, parity);
+    auto shade = [&](auto kernel) { launch_chained(kernel, grid((const void*)kernel, bs), bs, st, b, one, parity); };
+    launch_chained(engine_extend_kernel<kOne>, grid((const void*)engine_extend_kernel<kOne>, be), be, st, b, one, parity);
     const bool lights = !kOne || one.P.useLights;
     if (b.shadeThreadsPerSm == 512)
         lights ? shade(engine_shade_kernel<kOne, 512>) : shade(engine_shade_kernel<kOne, 512, false>);
@@ -976,7 +1012,7 @@ void bounce(const EngineBuffers& b, const EngineJob& one, int parity, int n, cud
         lights ? shade(engine_shade_kernel<kOne, 1024>) : shade(engine_shade_kernel<kOne, 1024, false>);
     else
         shade(engine_shade_kernel<kOne, 0>);
-    engine_shadow_kernel<kOne><<<grid((const void*)engine_shadow_kernel<kOne>, bw), bw, 0, st>>>(b, one, parity);
+    launch_chained(engine_shadow_kernel<kOne>, grid((const void*)engine_shadow_kernel<kOne>, bw), bw, st, b, one, parity);
 }
 
 template <bool kOne>
@@ -989,8 +1025,8 @@ void step(const EngineBuffers& b, const EngineJob& one, int parity, cudaStream_t
 template <bool kOne>
 void drain(const EngineBuffers& b, const EngineJob& one, int parity, int n, int limit, cudaStream_t st)
 {
-    engine_drain_kernel<kOne><<<full_grid((const void*)engine_drain_kernel<kOne>, kRunBlock, (long long)n * 32), kRunBlock, 0,
-                                st>>>(b, one, parity, limit);
+    launch_chained(engine_drain_kernel<kOne>, full_grid((const void*)engine_drain_kernel<kOne>, kRunBlock, (long long)n * 32),
+                   kRunBlock, st, b, one, parity, limit);
 }
 
 template <bool kOne>
@@ -1013,14 +1049,14 @@ int launch_frame_run(const EngineBuffers& b0, const EngineJob& one, const Engine
     {
         b.ps.L = radiance;
         auto direct = [&](auto kernel) {
-            kernel<<<full_grid((const void*)kernel, kRunBlock, (long long)n * 32), kRunBlock, 0, st>>>(b, one, first, table,
-                                                                                                      numPasses, n);
+            launch_chained(kernel, full_grid((const void*)kernel, kRunBlock, (long long)n * 32), kRunBlock, st, b, one, first,
+                           (const EnginePass*)table, numPasses, n);
         };
         one.P.useLights ? direct(engine_direct_kernel<true>) : direct(engine_direct_kernel<false>);
         return (int)cudaGetLastError();
     }
-    engine_start_kernel<<<full_grid((const void*)engine_start_kernel, 256, n), 256, 0, st>>>(b, one.P, first, table,
-                                                                                             numPasses, n);
+    launch_chained(engine_start_kernel, full_grid((const void*)engine_start_kernel, 256, n), 256, st, b, one.P, first, table,
+                   numPasses, n);
     const int bounces = std::min(one.P.maxDepth, kRunBounces);
     for (int k = 0; k < bounces; ++k)
     {
@@ -1036,8 +1072,8 @@ int launch_engine_accumulate_run(const Params& P, const EnginePass* table, int c
 {
     const int B = 256;
     const long long pix = (long long)P.width * P.height;
-    engine_accumulate_run_kernel<<<full_grid((const void*)engine_accumulate_run_kernel, B, pix), B, 0, st>>>(
-        P.width, P.height, P.tileW, P.tileH, table, chunks, tilesX, tilesY, accum, accum64);
+    launch_chained(engine_accumulate_run_kernel, full_grid((const void*)engine_accumulate_run_kernel, B, pix), B, st, P.width,
+                   P.height, P.tileW, P.tileH, table, chunks, tilesX, tilesY, accum, accum64);
     return (int)cudaGetLastError();
 }
 
@@ -1064,8 +1100,8 @@ int launch_engine_accumulate(const Params& P, const EnginePass& pass, float4* ac
 {
     const int B = 256;
     const long long pix = (long long)pass.visW * pass.visH;
-    engine_accumulate_kernel<<<full_grid((const void*)engine_accumulate_kernel, B, pix), B, 0, st>>>(
-        P.width, P.tileW, P.tileH, pass, accum, accum64);
+    launch_chained(engine_accumulate_kernel, full_grid((const void*)engine_accumulate_kernel, B, pix), B, st, P.width, P.tileW,
+                   P.tileH, pass, accum, accum64);
     return (int)cudaGetLastError();
 }
 }
