@@ -41,14 +41,15 @@ constexpr int kMaxTraversalSteps = 1 << 22;
 
 // Device error bits (LF_DEVERR_*) are the ones of the C ABI, OR-ed into a status word.
 
-struct DevLight
+struct alignas(16) DevLight   // in groups of 16 bytes, which come in one load each
 {
-    float pos[3], emission[3], u[3], v[3];
-    float radius, area, type;
-    float normal[3];        // normalize(cross(u, v))
-    float planeW;           // dot(normal, pos)
-    float us[3], vs[3];     // u / dot(u,u), v / dot(v,v)
-    float pad[3];
+    float pos[3], radius;
+    float emission[3], area;
+    float u[3], type;
+    float v[3], planeW;     // planeW: dot(normal, pos)
+    float normal[3], pad0;  // normalize(cross(u, v))
+    float us[3], pad1;      // u / dot(u,u)
+    float vs[3], pad2;      // v / dot(v,v)
 };
 
 // Wide nodes collapsed from the reference's binary tree (see traverse_wide): per node

@@ -198,16 +198,24 @@ struct SurfaceGeom
 
 __device__ __forceinline__ SurfaceGeom surface_geom(const ShadeScene& S, v3 o, v3 d, float t, int inst, int prim)
 {
-    float m[12];
-    int root, matId;
-    load_instance(S.trav.instances + (size_t)inst * 4, m, &root, &matId);
     const ShadeInstance& SI = S.inst[inst];
-    v3 ro = xform(m, o, 1.0f), rd = xform(m, d, 0.0f);
+    // an identity transform changes nothing but a component of -0, which its sums make +0
+    v3 ro = o + v3(0.0f), rd = d + v3(0.0f);
+    const bool identity = SI.identity != 0;
+    if (!identity)
+    {
+        float m[12];
+        int root, matId;
+        load_instance(S.trav.instances + (size_t)inst * 4, m, &root, &matId);
+        ro = xform(m, o, 1.0f);
+        rd = xform(m, d, 0.0f);
+    }
     float u, v;
     tri_hit(S.trav.tris + (size_t)prim * 3, ro, rd, &u, &v);
     float bw = 1.0f - u - v;
     SurfaceGeom g;
-    g.fhp = xform(SI.fwd, ro + rd * t, 1.0f);
+    const v3 hp = ro + rd * t;
+    g.fhp = identity ? hp + v3(0.0f) : xform(SI.fwd, hp, 1.0f);
     int4 vi = S.vertIndices[prim];
     float4 n1 = S.normals[vi.x], n2 = S.normals[vi.y], n3 = S.normals[vi.z];
     float w0 = S.vertices[vi.x].w, w1 = S.vertices[vi.y].w, w2 = S.vertices[vi.z].w;

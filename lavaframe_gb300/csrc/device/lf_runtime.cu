@@ -689,6 +689,9 @@ lf_status encode_instances(lf_ctx* c, const lf_scene_view* v, const RefNode* nod
             for (int r = 0; r < 3; ++r) s.fwd[col * 3 + r] = M[col * 4 + r];
         lfc::normal_matrix(M, s.nrm);
         s.material = mat;
+        const float ident[12] = {1, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0};
+        const float inv12[12] = {inv[0], inv[1], inv[2], inv[4], inv[5], inv[6], inv[8], inv[9], inv[10], inv[12], inv[13], inv[14]};
+        s.identity = std::memcmp(s.fwd, ident, sizeof ident) == 0 && std::memcmp(inv12, ident, sizeof ident) == 0 ? 1 : 0;
         // class of the material's shading code (Material.h layout: metallic [8], transmission
         // [16], texture ids [24..27]) for the engine's sort-by-material
         const float* mp = v->materials + (size_t)mat * 28;
