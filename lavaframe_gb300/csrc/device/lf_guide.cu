@@ -785,21 +785,45 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    const size_t qf = (size_t)n * kSampleFloats;
-    lf_status st = ensure_scratch(gd, qf + (size_t)n * (kMixFloats + 1));
-    if (st != LF_OK) return st;
-    float* dq = gd->scratch;
-    float* dmix = gd->scratch + qf;
-    float* dpdf = dmix + (size_t)n * kMixFloats;
-    cudaMemcpyAsync(dq, queries, qf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-    const int ie = gd->tensorPath ? launch_infer_tc(gd->net, dq, nullptr, n, dmix, c->d_status, c->stream)
-                                  : launch_infer(gd->net, dq, nullptr, n, dmix, c->stream);
+    const size_t qf = (size_t)n * kSampleFloats, mf = (size_t)n * kMixFloats;
+    // Small batches are read from and written to the page-locked staging block by the kernel: one
+    // launch and one wait (a copy to or from pageable memory costs 10 us whatever its size): 100
+    // queries 57 -> 34 us, 1000 65 -> 54.
+    const bool staged = (qf + mf + n) * sizeof(float) <= kStageBytes && ensure_stage(c);
+    if (!staged)
+    {
+        lf_status st = ensure_scratch(gd, qf + mf + n);
+        if (st != LF_OK) return st;
+    }
+    float* const hq = reinterpret_cast<float*>(c->stage);
+    float* const dq = staged ? reinterpret_cast<float*>(c->d_stage) : gd->scratch;
+    float* const dmix = dq + qf;
+    float* const dpdf = dmix + mf;
+    if (staged)
+        std::memcpy(hq, queries, qf * sizeof(float));
+    else
+        cudaMemcpyAsync(dq, queries, qf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    int ie;
+    if (gd->tensorPath)
+        ie = launch_infer_tc(gd->net, dq, nullptr, n, dmix, c->d_status, c->stream, dpdf);
+    else
+    {
+        ie = launch_infer(gd->net, dq, nullptr, n, dmix, c->stream);
+        if (!ie) guide_pdf_kernel<<<grid_blocks(n, 256), 256, 0, c->stream>>>(dmix, dq, n, dpdf);
+    }
     if (ie) return cuda_fail(c, (cudaError_t)ie, "guide inference launch");
-    guide_pdf_kernel<<<grid_blocks(n, 256), 256, 0, c->stream>>>(dmix, dq, n, dpdf);
-    if (mix) cudaMemcpyAsync(mix, dmix, (size_t)n * kMixFloats * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    if (pdf) cudaMemcpyAsync(pdf, dpdf, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    if (!staged)
+    {
+        if (mix) cudaMemcpyAsync(mix, dmix, mf * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+        if (pdf) cudaMemcpyAsync(pdf, dpdf, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    }
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide eval");
+    if (staged)
+    {
+        if (mix) std::memcpy(mix, hq + qf, mf * sizeof(float));
+        if (pdf) std::memcpy(pdf, hq + qf + mf, (size_t)n * sizeof(float));
+    }
     return check_device(c);
 }
 }

@@ -231,7 +231,7 @@ __device__ __forceinline__ bool group_sync_or(int id, bool v)
 // stepping by gridDim.x * kInferGroups, and synchronises on its own named barrier (1 + g), so
 // that one group's MMAs and waits overlap the other's encoding and epilogue.
 __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
-    guide_infer_tc_kernel(Net net, const float* queries, int n, const int* nDev, float* mix, uint32_t* status)
+    guide_infer_tc_kernel(Net net, const float* queries, int n, const int* nDev, float* mix, float* pdf, uint32_t* status)
 {
     if (nDev) n = *nDev;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -243,12 +243,12 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(bars + kInferGroups);
     const uint32_t mbar = smem_addr(bars + grp);
 
-    // weights [out][in] of the four layers -> B operands in core-matrix layout
-    for (int i = tid; i < kWeights; i += kInferThreads)
+    // weights [out][in] of the four layers -> B operands in core-matrix layout, 8 values at a time
+    for (int i = tid; i < kWeights / 8; i += kInferThreads)
     {
-        const int l = i < 3 * 4096 ? i >> 12 : 3;
-        const int r = (i - l * 4096) >> 6, k = (i - l * 4096) & 63;
-        *reinterpret_cast<__half*>(sW + l * kLayerBytes + cm_offset(r, k)) = net.W[i];
+        const int l = i < 3 * 512 ? i >> 9 : 3;
+        const int r = (i - l * 512) >> 3, k = ((i - l * 512) & 7) * 8;
+        *reinterpret_cast<uint4*>(sW + l * kLayerBytes + cm_offset(r, k)) = reinterpret_cast<const uint4*>(net.W)[i];
     }
     if (warp == 0)
     {
@@ -279,13 +279,17 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
     {
         const int q = tile * kTcRows + row;
         const bool valid = q < n;
+        float dir[3];
         {
-            // position, outgoing direction and normal in three 16-byte loads (records are 64 bytes apart)
+            // position, outgoing direction, normal and direction in three 16-byte loads (records are
+            // 64 bytes apart)
             float rec[12];
             const float4* src = reinterpret_cast<const float4*>(queries + (size_t)(valid ? q : 0) * kSampleFloats);
 #pragma unroll
             for (int k = 0; k < 3; ++k) *reinterpret_cast<float4*>(rec + 4 * k) = src[k];
             encode_row_direct(net, rec, valid, sA, row);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) dir[k] = rec[9 + k];
         }
         for (int layer = 0; layer < 4; ++layer)
         {
@@ -345,8 +349,9 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
         }
         const float invEs = 1.f / es;
         float* dst = mix + (size_t)(valid ? q : 0) * kMixFloats;
-        float cum = 0.f;
-        // four lobes at a time: 20 values in five 16-byte stores
+        float cum = 0.f, density = 0.f, prev = 0.f;
+        // four lobes at a time: 20 values in five 16-byte stores; the density of the record's direction
+        // on request, as mix_pdf sums it
 #pragma unroll
         for (int half = 0; half < kLobes; half += 4)
         {
@@ -369,6 +374,13 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
                 o[5 * i + 2] = mu[2];
                 o[5 * i + 3] = k;
                 o[5 * i + 4] = half + i == kLobes - 1 ? 1.f : cum;
+                if (pdf)
+                {
+                    const float pi = o[5 * i + 4] - prev;
+                    prev = o[5 * i + 4];
+                    const float dot = mu[0] * dir[0] + mu[1] * dir[1] + mu[2] * dir[2];
+                    density += pi * vmf_norm(k) * __expf(k * (dot - 1.f));
+                }
             }
             if (valid)
 #pragma unroll
@@ -376,6 +388,7 @@ __global__ void __launch_bounds__(kInferThreads, kInferCtasPerSm)
                     *reinterpret_cast<float4*>(dst + 5 * half + 4 * k) =
                         make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
         }
+        if (pdf && valid) pdf[q] = density;
     }
     fence_before_sync();
     __syncthreads();
@@ -711,7 +724,7 @@ int launch_train_tc(const Net& net, const float* samples, int n, float* gW, floa
 }
 
 int launch_infer_tc(const Net& net, const float* queries, const int* nDev, int cap, float* mix, uint32_t* status,
-                    cudaStream_t st)
+                    cudaStream_t st, float* pdf)
 {
     static bool attr = false;
     if (!attr)
@@ -727,7 +740,7 @@ int launch_infer_tc(const Net& net, const float* queries, const int* nDev, int c
     // SM's 512, so no allocation waits
     const int tiles = (cap + kTcRows - 1) / kTcRows;
     const int blocks = std::max(1, std::min(sms * kInferCtasPerSm, (tiles + kInferGroups - 1) / kInferGroups));
-    guide_infer_tc_kernel<<<blocks, kInferThreads, kTcSmem, st>>>(net, queries, cap, nDev, mix, status);
+    guide_infer_tc_kernel<<<blocks, kInferThreads, kTcSmem, st>>>(net, queries, cap, nDev, mix, pdf, status);
     return (int)cudaGetLastError();
 }
 }
