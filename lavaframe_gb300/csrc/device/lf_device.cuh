@@ -922,7 +922,17 @@ __device__ __forceinline__ bool wide_step(const DevScene& S, WideRay& w, int* st
     return false;
 }
 
-template <bool kAny>
+// Node steps a lane takes before its warp visits the leaves and instances that its lanes have come to.
+// With one, nearly every round of a warp runs both kinds of step for part of its lanes; with more, lanes
+// at a leaf wait while the others go on. Occlusion queries, whose steps are short, gain with three: 4M
+// rays against random triangles 3.71 -> 3.49 ms, 2M rays in a room 227 -> 207 us, the Cornell box
+// 182 -> 170 (two 3.48 / 219 / 173, four 3.54 / 198 / 165, until the next leaf 4.36 / 170 / 173). Closest hits of
+// random rays lose (two steps: room 489 -> 505, spheres 621 -> 643), those of camera and bounce rays in
+// the step kernels gain with two: spheres 1080p x 8 12.73 -> 12.52 ms, room 2M paths 3.34 -> 3.33.
+constexpr int kAnyNodeSteps = 3;
+constexpr int kPathNodeSteps = 2;
+
+template <bool kAny, int kNodeSteps>
 __device__ __forceinline__ uint32_t traverse_wide(const DevScene& S, v3 o, v3 d, float* tBest, Hit* out)
 {
     bool fast;
@@ -934,14 +944,26 @@ __device__ __forceinline__ uint32_t traverse_wide(const DevScene& S, v3 o, v3 d,
     int stack[kWideStack + kWide];   // the overflow test follows a node's pushes
     wide_init(S, w, o, d, winvd, *tBest);
     Hit h = *out;
-    while (!wide_step<kAny>(S, w, stack, h)) {}
+    if constexpr (kNodeSteps > 1)
+    {
+        bool done = false;
+        while (!done)
+        {
+#pragma unroll
+            for (int k = 0; k < kNodeSteps; ++k)
+                if (!done && w.code >= 0) done = wide_step<kAny>(S, w, stack, h);
+            if (!done && w.code < 0) done = wide_step<kAny>(S, w, stack, h);
+        }
+    }
+    else
+        while (!wide_step<kAny>(S, w, stack, h)) {}
     *out = h;
     *tBest = w.t;
     return w.err;
 }
 
 // Closest hit: analytic lights first (closest_hit.glsl:13-67), then the BVH.
-template <bool kStats>
+template <bool kStats, int kNodeSteps = 1>
 __device__ __forceinline__ uint32_t closest_hit(const DevScene& S, v3 o, v3 d, float tInit, bool useLights,
                                                 Hit* out, TraceStats* st)
 {
@@ -971,7 +993,7 @@ __device__ __forceinline__ uint32_t closest_hit(const DevScene& S, v3 o, v3 d, f
             }
         }
     }
-    uint32_t err = (!kStats && S.wnodes && S.wideOn) ? traverse_wide<false>(S, o, d, &t, out)
+    uint32_t err = (!kStats && S.wnodes && S.wideOn) ? traverse_wide<false, kNodeSteps>(S, o, d, &t, out)
                                                       : traverse<false, kStats>(S, o, d, &t, out, st);
     out->t = t;
     return err;
@@ -1004,7 +1026,7 @@ __device__ __forceinline__ uint32_t any_hit(const DevScene& S, v3 o, v3 d, float
         }
     }
     float t = maxDist;
-    uint32_t err = (!kStats && S.wnodes && S.wideOn) ? traverse_wide<true>(S, o, d, &t, out)
+    uint32_t err = (!kStats && S.wnodes && S.wideOn) ? traverse_wide<true, kAnyNodeSteps>(S, o, d, &t, out)
                                                      : traverse<true, kStats>(S, o, d, &t, out, st);
     *occluded = out->prim >= 0;
     out->t = *occluded ? t : kInfinity;

@@ -494,7 +494,7 @@ __global__ void __maxnreg__(72) engine_extend_kernel(EngineBuffers b, EngineJob 
             const ShadeInstance* sinst;
             if constexpr (kOne)
             {
-                err = closest_hit<false>(one.S.trav, f3(o4), f3(d4), kInfinity, one.P.useLights != 0, &h, nullptr);
+                err = closest_hit<false, kPathNodeSteps>(one.S.trav, f3(o4), f3(d4), kInfinity, one.P.useLights != 0, &h, nullptr);
                 sinst = one.S.inst;
             }
             else
@@ -502,7 +502,7 @@ __global__ void __maxnreg__(72) engine_extend_kernel(EngineBuffers b, EngineJob 
                 const int w = reinterpret_cast<const int*>(b.ps.info)[4 * p + 3];
                 const EngineJob& J = b.jobs[job_of(w)];
                 const DevScene T = J.S.trav;
-                err = closest_hit<false>(T, f3(o4), f3(d4), kInfinity, J.P.useLights != 0, &h, nullptr);
+                err = closest_hit<false, kPathNodeSteps>(T, f3(o4), f3(d4), kInfinity, J.P.useLights != 0, &h, nullptr);
                 sinst = J.S.inst;
             }
             b.ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));

@@ -71,7 +71,7 @@ __global__ void __maxnreg__(72) extend_kernel(ShadeScene S, Params P, PathSoA ps
         int p = queue[i];
         float4 o4 = ps.o[p], d4 = ps.d[p];
         Hit h;
-        uint32_t err = closest_hit<false>(S.trav, f3(o4), f3(d4), kInfinity, lights, &h, nullptr);
+        uint32_t err = closest_hit<false, kPathNodeSteps>(S.trav, f3(o4), f3(d4), kInfinity, lights, &h, nullptr);
         ps.hit[p] = make_float4(h.t, __int_as_float(h.inst), __int_as_float(h.prim), __int_as_float(h.light));
         set_error(status, err);
     }
