@@ -194,7 +194,7 @@ bool ensure_stage(lf_ctx* c);
 // The copy streams and events of calls that overlap copies with kernels, made on first use.
 cudaError_t ensure_chunk_streams(lf_ctx* c);
 // The colour channels of n padded pixels into host memory, after the stream's work (synchronises).
-cudaError_t copy_rgb(lf_ctx* c, const float4* src, size_t n, float* rgb);
+cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb);
 
 struct RefNode
 {

@@ -1309,15 +1309,15 @@ namespace lfrt
 // The three colour channels of n padded pixels in the caller's buffer: packed on the device and
 // copied there directly (copying the padded pixels for the host to repack took 2.4 ms more of a
 // 1920 x 1080 x 16 render: 30.7 -> 28.3 ms).
-cudaError_t copy_rgb(lf_ctx* c, const float4* src, size_t n, float* rgb)
+cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb)
 {
     float* packed = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&packed, n * 3 * sizeof(float), c->stream);
+    cudaError_t e = cudaMallocAsync((void**)&packed, n * 3 * sizeof(float), st);
     if (e != cudaSuccess) return e;
-    e = (cudaError_t)launch_pack_rgb(src, (long long)n, packed, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, packed, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-    cudaFreeAsync(packed, c->stream);
-    const cudaError_t s = cudaStreamSynchronize(c->stream);
+    e = (cudaError_t)launch_pack_rgb(src, (long long)n, packed, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, packed, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
+    cudaFreeAsync(packed, st);
+    const cudaError_t s = cudaStreamSynchronize(st);
     return e == cudaSuccess ? s : e;
 }
 
@@ -1732,7 +1732,7 @@ lf_status lf_frame_read_accum(lf_frame* f, float* rgb)
     lf_ctx* c = f->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    const cudaError_t e = copy_rgb(c, f->accum, (size_t)f->W * f->H, rgb);
+    const cudaError_t e = copy_rgb(c->stream, f->accum, (size_t)f->W * f->H, rgb);
     if (e != cudaSuccess) return cuda_fail(c, e, "accum readback");
     return check_device(c);
 }

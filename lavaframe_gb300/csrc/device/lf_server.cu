@@ -84,6 +84,7 @@ struct lf_server
     lf_server_stats stats{};
     unsigned long long ctrBase[4] = {0, 0, 0, 0};   // engine counters at creation
     std::string err;
+    cudaStream_t readStream = nullptr;   // job readbacks
 };
 
 namespace
@@ -306,13 +307,28 @@ void scheduler(lf_server* s)
         if (running == 0)
         {
             bool pending = false;
+            cudaEvent_t last = nullptr;
             for (auto& kv : s->jobs)
-                if (kv.second.state == LF_JOB_RUNNING) pending = true;
+                if (kv.second.state == LF_JOB_RUNNING)
+                {
+                    pending = true;
+                    if (kv.second.doneEvent) last = kv.second.doneEvent;
+                }
             if (s->stop && !pending) break;
             if (!pending && s->queue.empty())
+            {
                 s->cv.wait(lk);
-            else
-                s->cv.wait_for(lk, std::chrono::microseconds(200));
+                continue;
+            }
+            if (last)
+            {
+                // only accumulations are left: wait for one (a running job's event outlives it)
+                lk.unlock();
+                const cudaError_t we = cudaEventSynchronize(last);
+                lk.lock();
+                if (we == cudaSuccess) continue;
+            }
+            s->cv.wait_for(lk, std::chrono::microseconds(200));
             continue;
         }
         // 3. one pair of steps (unlocked while the GPU runs)
@@ -378,6 +394,11 @@ lf_status lf_server_create(lf_ctx* c, const lf_server_config* cfg, lf_server** o
         std::lock_guard<std::recursive_mutex> g(c->mu);
         cudaSetDevice(c->device);
         lf_status st = engine_get(c, &s->engine);
+        if (st == LF_OK)
+        {
+            const cudaError_t e = cudaStreamCreateWithFlags(&s->readStream, cudaStreamNonBlocking);
+            if (e != cudaSuccess) st = cuda_fail(c, e, "server stream");
+        }
         if (st != LF_OK)
         {
             delete s;
@@ -392,6 +413,7 @@ lf_status lf_server_create(lf_ctx* c, const lf_server_config* cfg, lf_server** o
     }
     if (s->deviceBytes > s->cfg.memory_budget)
     {
+        cudaStreamDestroy(s->readStream);
         delete s;
         return fail(c, LF_ERR_BUDGET, "the engine pool alone exceeds the memory budget");
     }
@@ -496,10 +518,13 @@ lf_status lf_server_read(lf_server* s, int64_t job_id, float* rgb)
     ServerJob& j = it->second;
     if (j.state != LF_JOB_DONE) return fail(s->ctx, LF_ERR_STATE, "job not done");
     lf_ctx* c = s->ctx;
-    std::lock_guard<std::recursive_mutex> g(c->mu);
     cudaSetDevice(c->device);
-    const cudaError_t e = copy_rgb(c, j.accum, (size_t)j.params.width * j.params.height, rgb);
-    return e == cudaSuccess ? LF_OK : cuda_fail(c, e, "job readback");
+    // a done job's image is complete (its event has passed), so it is read on a stream of its own, beside
+    // the step pair that the scheduler has in flight
+    const cudaError_t e = copy_rgb(s->readStream, j.accum, (size_t)j.params.width * j.params.height, rgb);
+    if (e == cudaSuccess) return LF_OK;
+    std::lock_guard<std::recursive_mutex> g(c->mu);
+    return cuda_fail(c, e, "job readback");
 }
 
 lf_status lf_server_release_job(lf_server* s, int64_t job_id)
@@ -585,6 +610,7 @@ lf_status lf_server_destroy(lf_server* s)
     for (auto& kv : s->scenes)
         if (kv.second.dev) lf_scene_release(kv.second.dev);
     cudaStreamSynchronize(c->stream);
+    cudaStreamDestroy(s->readStream);
     delete s;
     return LF_OK;
 }
