@@ -705,21 +705,33 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats + kGridParams);
+    const size_t gridBytes = (size_t)kGridParams * sizeof(float);
+    // samples are read and grid gradients written where they are if the kernels can: 16,384 samples
+    // 97 -> 88 us, a first call into fresh buffers 255 -> 130
+    const bool directIn = direct_host(c, samples, (size_t)n * kSampleFloats * sizeof(float), false);
+    const bool directGrid = disjoint(samples, (size_t)n * kSampleFloats * sizeof(float), dgrid, gridBytes) &&
+                            direct_host(c, dgrid, gridBytes, true);
+    lf_status st = ensure_scratch(gd, (directIn ? 0 : (size_t)n * kSampleFloats) + (directGrid ? 0 : kGridParams));
     if (st != LF_OK) return st;
     if (!ensure_stage(c)) return fail(c, LF_ERR_OOM, "guide gradient staging");
-    float* const outGrid = gd->scratch + (size_t)n * kSampleFloats;   // samples are 16 floats: aligned
+    float* const outGrid = directGrid ? dgrid : gd->scratch;
+    const float* in = samples;
     // the small results go to page-locked memory, which saves two copies' latencies
     static_assert((kWeights + 1) * sizeof(float) <= kStageBytes, "weight gradients and the loss fit the staging block");
     float* const hW = reinterpret_cast<float*>(c->stage);
     float* const dW = reinterpret_cast<float*>(c->d_stage);
-    cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    if (!directIn)
+    {
+        float* const copy = gd->scratch + (directGrid ? 0 : kGridParams);   // 16-byte aligned
+        cudaMemcpyAsync(copy, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+        in = copy;
+    }
     cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);      // training steps leave theirs
-    st = run_gradients(gd, gd->scratch, n);
+    st = run_gradients(gd, in, n);
     if (st != LF_OK) return st;
     guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(
         gd->wGrad, gd->gGrad, gd->dLoss, 1.f / (float)n, dW, outGrid, dW + kWeights);
-    cudaMemcpyAsync(dgrid, outGrid, (size_t)kGridParams * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    if (!directGrid) cudaMemcpyAsync(dgrid, outGrid, gridBytes, cudaMemcpyDeviceToHost, c->stream);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide gradients");
     std::memcpy(dweights, hW, kWeights * sizeof(float));
@@ -755,12 +767,21 @@ lf_status lf_guide_train(lf_guide* gd, const float* samples, int32_t n, float lr
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats);
-    if (st != LF_OK) return st;
-    cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    const float* in = samples;
+    if (!direct_host(c, samples, (size_t)n * kSampleFloats * sizeof(float), false))
+    {
+        lf_status st = ensure_scratch(gd, (size_t)n * kSampleFloats);
+        if (st != LF_OK) return st;
+        cudaMemcpyAsync(gd->scratch, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+        in = gd->scratch;
+    }
     cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);
-    st = lf_guide_train_device(gd, gd->scratch, n, lr);
-    if (st != LF_OK) return st;
+    lf_status st = lf_guide_train_device(gd, in, n, lr);
+    if (st != LF_OK)
+    {
+        cudaStreamSynchronize(c->stream);   // no kernel may still read the caller's samples
+        return st;
+    }
     if (loss)
     {
         double sum = 0.0;
@@ -786,23 +807,40 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
     const size_t qf = (size_t)n * kSampleFloats, mf = (size_t)n * kMixFloats;
-    // Small batches are read from and written to the page-locked staging block by the kernel: one
-    // launch and one wait (a copy to or from pageable memory costs 10 us whatever its size): 100
-    // queries 57 -> 34 us, 1000 65 -> 54.
+    // A copy to or from pageable memory costs 10 us whatever its size. So small batches go over the
+    // page-locked staging block (100 queries 57 -> 34 us, 1000 65 -> 52), and on a coherent host the
+    // kernel reads up to kDirectQueries queries (8,000 queries 76 -> 58 us, 33,000 109 -> 94; with
+    // 100,000 the kernel waits for them: 225 us against 212) and writes the densities (100,000: 213 ->
+    // 204 us) where they are. Mixtures are written in 20-byte lobes by lanes that are 160 bytes
+    // apart: copied (100,000 direct: 408 us).
+    constexpr int kDirectQueries = 1 << 15;
     const bool staged = (qf + mf + n) * sizeof(float) <= kStageBytes && ensure_stage(c);
+    const bool directIn = !staged && n <= kDirectQueries && direct_host(c, queries, qf * sizeof(float), false);
+    const bool directPdf = !staged && pdf && disjoint(queries, qf * sizeof(float), pdf, (size_t)n * sizeof(float)) &&
+                           direct_host(c, pdf, (size_t)n * sizeof(float), true, 4);
     if (!staged)
     {
-        lf_status st = ensure_scratch(gd, qf + mf + n);
+        lf_status st = ensure_scratch(gd, (directIn ? 0 : qf) + mf + n);
         if (st != LF_OK) return st;
     }
-    float* const hq = reinterpret_cast<float*>(c->stage);
-    float* const dq = staged ? reinterpret_cast<float*>(c->d_stage) : gd->scratch;
-    float* const dmix = dq + qf;
-    float* const dpdf = dmix + mf;
-    if (staged)
-        std::memcpy(hq, queries, qf * sizeof(float));
-    else
-        cudaMemcpyAsync(dq, queries, qf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+    float* next = staged ? reinterpret_cast<float*>(c->d_stage) : gd->scratch;
+    auto take = [&](size_t floats) {
+        float* p = next;
+        next += floats;
+        return p;
+    };
+    const float* dq = queries;
+    if (!directIn)
+    {
+        float* copy = take(qf);
+        if (staged)
+            std::memcpy(c->stage, queries, qf * sizeof(float));
+        else
+            cudaMemcpyAsync(copy, queries, qf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+        dq = copy;
+    }
+    float* const dmix = take(mf);
+    float* const dpdf = directPdf ? pdf : take((size_t)n);
     int ie;
     if (gd->tensorPath)
         ie = launch_infer_tc(gd->net, dq, nullptr, n, dmix, c->d_status, c->stream, dpdf);
@@ -815,14 +853,15 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
     if (!staged)
     {
         if (mix) cudaMemcpyAsync(mix, dmix, mf * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
-        if (pdf) cudaMemcpyAsync(pdf, dpdf, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+        if (pdf && !directPdf) cudaMemcpyAsync(pdf, dpdf, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     }
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide eval");
     if (staged)
     {
-        if (mix) std::memcpy(mix, hq + qf, mf * sizeof(float));
-        if (pdf) std::memcpy(pdf, hq + qf + mf, (size_t)n * sizeof(float));
+        const char* base = c->d_stage;
+        if (mix) std::memcpy(mix, c->stage + (reinterpret_cast<char*>(dmix) - base), mf * sizeof(float));
+        if (pdf) std::memcpy(pdf, c->stage + (reinterpret_cast<char*>(dpdf) - base), (size_t)n * sizeof(float));
     }
     return check_device(c);
 }

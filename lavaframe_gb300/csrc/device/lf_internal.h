@@ -63,6 +63,7 @@ struct lf_ctx
     size_t binCap = 0;
     uint32_t* binHist = nullptr;
     unsigned long long* binNext = nullptr;   // fetch counter and blocks done, zero between launches
+    bool hostDirect = false;                 // kernels may address the host's own memory (direct_host)
     char* stage = nullptr;                   // page-locked staging block (ensure_stage)
     char* d_stage = nullptr;                 // its device address
     lfrt::EngineHost* engine = nullptr;   // multi-job engine, created on first use
@@ -186,6 +187,21 @@ inline lf_status check_device(lf_ctx* c)
 // Kernel parameters of one render (lf_render_params + scene facts); tile fields cover the
 // whole frame unless the parameters set a tile size.
 void fill_params(Params& P, const lf_render_params* p, const lf_scene* sc);
+
+// Whether a kernel may read (or write) the caller's buffer itself. On a coherent host (Grace: the GPU
+// walks the host's page tables) any memory of the process can be addressed, and what the kernel moves
+// over C2C is hidden behind its work, which a copy before or after it is not. The pages are
+// brought in first: that tells a range that isn't mapped (or not writable) from one that is before
+// a kernel meets it - such a range takes the copy path and its errors - and fresh pages cost a third
+// less than when the GPU faults them in one by one (32 MB: 0.78 ms, 1.16 faulted, 0.97 by copy).
+// Buffers must be aligned for the kernel's words; on other hosts everything is copied.
+bool direct_host(const lf_ctx* c, const void* p, size_t bytes, bool write, size_t align = 16);
+// Inputs and results that overlap go through copies.
+inline bool disjoint(const void* a, size_t na, const void* b, size_t nb)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x + na <= y || y + nb <= x;
+}
 
 // Page-locked staging of small results and queries, mapped for the kernels (c->stage, c->d_stage);
 // false when there is none.

@@ -11,6 +11,9 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "lf_engine.h"
 #include "lf_engine_host.h"
 #include "lf_pixel.h"
@@ -38,6 +41,9 @@ lf_status lf_ctx_create(int32_t device, lf_ctx** out)
         return e == cudaErrorMemoryAllocation ? LF_ERR_OOM : LF_ERR_CUDA;
     }
     c->h_status[0] = c->h_status[1] = 0;
+    int coherent = 0;
+    if (cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) == cudaSuccess)
+        c->hostDirect = coherent != 0;
     // frame buffers and pass radiance come from the stream-ordered pool; keep up to 8 GB of it cached
     // between calls instead of handing it back to CUDA at every synchronisation
     cudaMemPool_t pool = nullptr;
@@ -1179,12 +1185,28 @@ void read_trace_stats(lf_ctx* c)
     for (int k = 0; k < 3; ++k) c->lastStats[k] = s[k];
 }
 
-// Copies the rays in, traces them and copies the results out, in `host_chunks` pieces: piece k
-// is copied in on copyIn, sorted and traced on the context stream once its copy is done, and
-// copied out on copyOut once traced, so copies of some pieces overlap the tracing of others.
-// When the results go to a mapped page-locked block of this context, the kernels write them
-// there and nothing is copied out. The context stream waits for the copy streams, and the
-// call returns after it.
+// Whether a host query is traced in input order, from and to the caller's buffers if the kernel can
+// address them (direct_host). Each ray is then read and each result written once and in turn, beside
+// the tracing of others; binned rays are gathered and their results scattered, which C2C takes badly
+// (1M closest hits on the Cornell box 0.65 against 0.48 ms), so those work on copies. Direct in
+// input order / copied and binned, us, on the Cornell box, a room, spheres, 1.3M, 2M and 5.2M random
+// triangles: 600k rays 167 / 317, 227 / 367, 254 / 418, 984 / 999, 1082 / 1039, 1415 / 1326; 4M rays
+// 799 / 1676, 1193 / 1996, 1263 / 2184, 5413 / 5576, 5968 / 5757, 8100 / 6971. Binning pays once
+// triangles and nodes outgrow the 129 MB L2. Occlusion, 12M rays: 10.6 / 11.7 ms on 2M triangles,
+// 11.8 / 12.2 on 5.2M; equal on 10.5M. Sizes that are not binned either way: 8,000 closest hits 53 ->
+// 31 us, 300,000 179 -> 104.
+constexpr int kDirectClosestTris = 1500000;
+bool direct_query(const lf_scene* sc, int64_t n, bool any, uint32_t flags)
+{
+    return any || (flags & LF_TRACE_UNSORTED) || !trace_sorts(n, any) || sc->view.trav.numTris <= kDirectClosestTris;
+}
+
+// Traces from and to the caller's buffers (direct_query), or copies the rays in, traces them and
+// copies the results out, in `host_chunks` pieces: piece k is copied in on copyIn, sorted and traced
+// on the context stream once its copy is done, and copied out on copyOut once traced, so copies of
+// some pieces overlap the tracing of others. When the results go to a mapped page-locked block of
+// this context, the kernels write them there and nothing is copied out. The context stream waits
+// for the copy streams, and the call returns after it.
 template <class Launch>
 lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void* out, size_t outElem, uint32_t flags,
                      Launch launch)
@@ -1209,7 +1231,7 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
         // there, so that the call is one launch and one wait
         char* s_out = c->stage + (size_t)n * 32;
         std::memcpy(c->stage, rays, (size_t)n * 32);
-        lf_status sst = launch(c->d_stage, c->d_stage + (size_t)n * 32, n);
+        lf_status sst = launch(c->d_stage, c->d_stage + (size_t)n * 32, n, 0);
         const lf_status dst = check_device(c);
         if (sst == LF_OK) sst = dst;
         if (sst == LF_OK) std::memcpy(out, s_out, (size_t)n * outElem);
@@ -1217,9 +1239,19 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
         return sst;
     }
     char* direct = mapped_range(c, out, (size_t)n * outElem);
+    const int K = host_chunks(c, n, flags);
+    if (c->hostChunks <= 1 && direct_query(sc, n, outElem == 1, flags) &&
+        disjoint(rays, (size_t)n * 32, out, (size_t)n * outElem) && direct_host(c, rays, (size_t)n * 32, false) &&
+        (direct || direct_host(c, out, (size_t)n * outElem, true)))
+    {
+        lf_status sst = launch((char*)const_cast<float*>(rays), direct ? direct : (char*)out, n, LF_TRACE_UNSORTED);
+        const lf_status dst = check_device(c);
+        if (sst == LF_OK) sst = dst;
+        if (sst == LF_OK && (flags & LF_TRACE_STATS)) read_trace_stats(c);
+        return sst;
+    }
     cudaError_t e = ensure(&c->scratchRays, &c->scratchRaysBytes, (size_t)n * 32);
     if (e == cudaSuccess && !direct) e = ensure(&c->scratchOut, &c->scratchOutBytes, (size_t)n * outElem);
-    const int K = host_chunks(c, n, flags);
     if (e == cudaSuccess && K > 1) e = ensure_chunk_streams(c);
     char* d_rays = (char*)c->scratchRays;
     char* d_out = direct ? direct : (char*)c->scratchOut;
@@ -1227,7 +1259,7 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
     if (e == cudaSuccess && K == 1)
     {
         e = cudaMemcpyAsync(d_rays, rays, (size_t)n * 32, cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess) st = launch(d_rays, d_out, n);
+        if (e == cudaSuccess) st = launch(d_rays, d_out, n, 0);
         if (e == cudaSuccess && st == LF_OK && !direct)
             e = cudaMemcpyAsync(out, d_out, (size_t)n * outElem, cudaMemcpyDeviceToHost, c->stream);
     }
@@ -1249,7 +1281,7 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
         {
             const int64_t lo = std::min(n, step * k), hi = k == K - 1 ? n : std::min(n, step * (k + 1));
             e = cudaStreamWaitEvent(c->stream, c->chunkIn[k], 0);
-            if (e == cudaSuccess && hi > lo) st = launch(d_rays + lo * 32, d_out + lo * outElem, hi - lo);
+            if (e == cudaSuccess && hi > lo) st = launch(d_rays + lo * 32, d_out + lo * outElem, hi - lo, 0);
             if (direct) continue;
             if (e == cudaSuccess && st == LF_OK) e = cudaEventRecord(c->chunkDone[k], c->stream);
             if (e == cudaSuccess && st == LF_OK) e = cudaStreamWaitEvent(c->copyOut, c->chunkDone[k], 0);
@@ -1283,15 +1315,15 @@ lf_status lf_ctx_set_host_chunks(lf_ctx* c, int32_t chunks)
 
 lf_status lf_trace_closest(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, lf_hit* hits, uint32_t flags)
 {
-    return trace_host(c, sc, rays, n, hits, sizeof(lf_hit), flags, [&](void* dr, void* dout, int64_t m) {
-        return lf_trace_closest_device(c, sc, dr, m, dout, flags);
+    return trace_host(c, sc, rays, n, hits, sizeof(lf_hit), flags, [&](void* dr, void* dout, int64_t m, uint32_t more) {
+        return lf_trace_closest_device(c, sc, dr, m, dout, flags | more);
     });
 }
 
 lf_status lf_trace_any(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, uint8_t* occ, uint32_t flags)
 {
-    return trace_host(c, sc, rays, n, occ, 1, flags, [&](void* dr, void* dout, int64_t m) {
-        return lf_trace_any_device(c, sc, dr, m, dout, flags);
+    return trace_host(c, sc, rays, n, occ, 1, flags, [&](void* dr, void* dout, int64_t m, uint32_t more) {
+        return lf_trace_any_device(c, sc, dr, m, dout, flags | more);
     });
 }
 
@@ -1306,16 +1338,29 @@ lf_status lf_trace_stats(const lf_ctx* c, uint64_t out3[3])
 extern "C++" {
 namespace lfrt
 {
+bool direct_host(const lf_ctx* c, const void* p, size_t bytes, bool write, size_t align)
+{
+#if defined(MADV_POPULATE_READ) && defined(MADV_POPULATE_WRITE)
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    if (!c->hostDirect || a % align) return false;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = a & ~(page - 1);
+    return madvise(reinterpret_cast<void*>(lo), a + bytes - lo, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) == 0;
+#else
+    return false;
+#endif
+}
+
 // The three colour channels of n padded pixels in the caller's buffer: packed on the device and
 // copied there directly (copying the padded pixels for the host to repack took 2.4 ms more of a
 // 1920 x 1080 x 16 render: 30.7 -> 28.3 ms).
 cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb)
 {
+    const size_t bytes = n * 3 * sizeof(float);
     float* packed = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&packed, n * 3 * sizeof(float), st);
+    cudaError_t e = cudaMallocAsync((void**)&packed, bytes, st);
     if (e != cudaSuccess) return e;
     e = (cudaError_t)launch_pack_rgb(src, (long long)n, packed, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, packed, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, packed, bytes, cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(packed, st);
     const cudaError_t s = cudaStreamSynchronize(st);
     return e == cudaSuccess ? s : e;

@@ -34,6 +34,7 @@ static_assert(kScanBlocks >= 1 && kScanBlocks <= 2 * kScanBlock, "bin scan cover
 // 626 / 709. Occlusion queries end early and write one byte per ray, which binning scatters: 4M
 // rays 4254 / 4460, 472 / 485, 1033 / 1048, 427 / 373; 16M rays 16.3 / 17.3, 1.89 / 1.87,
 // 3.96 / 3.86, 1.69 / 1.44 ms.
+// Queries of host buffers have a rule of their own (direct_query).
 constexpr long long kSortClosest = 1 << 19;
 constexpr long long kSortAny = 1 << 23;
 // 64^3 cells from here on, 32^3 below: 4M rays 4.94 / 4.97 ms on the random triangles, but 1.00 / 0.94,
