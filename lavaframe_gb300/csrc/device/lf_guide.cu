@@ -809,18 +809,21 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
     const size_t qf = (size_t)n * kSampleFloats, mf = (size_t)n * kMixFloats;
     // A copy to or from pageable memory costs 10 us whatever its size. So small batches go over the
     // page-locked staging block (100 queries 57 -> 34 us, 1000 65 -> 52), and on a coherent host the
-    // kernel reads up to kDirectQueries queries (8,000 queries 76 -> 58 us, 33,000 109 -> 94; with
-    // 100,000 the kernel waits for them: 225 us against 212) and writes the densities (100,000: 213 ->
-    // 204 us) where they are. Mixtures are written in 20-byte lobes by lanes that are 160 bytes
-    // apart: copied (100,000 direct: 408 us).
+    // kernel reads up to kDirectQueries queries and writes their mixtures where they are (5,000 queries 72
+    // -> 49 us, 32,768 107 -> 86; with 100,000 it waits for the queries, 225 us against 212, and the
+    // copy engine is the faster way for 16 MB of mixtures, 206 against 210), and the densities of any
+    // number (100,000: 213 -> 206 us).
     constexpr int kDirectQueries = 1 << 15;
     const bool staged = (qf + mf + n) * sizeof(float) <= kStageBytes && ensure_stage(c);
     const bool directIn = !staged && n <= kDirectQueries && direct_host(c, queries, qf * sizeof(float), false);
     const bool directPdf = !staged && pdf && disjoint(queries, qf * sizeof(float), pdf, (size_t)n * sizeof(float)) &&
                            direct_host(c, pdf, (size_t)n * sizeof(float), true, 4);
+    const bool directMix = !staged && n <= kDirectQueries && mix && gd->tensorPath &&
+                           disjoint(queries, qf * sizeof(float), mix, mf * sizeof(float)) &&
+                           direct_host(c, mix, mf * sizeof(float), true);
     if (!staged)
     {
-        lf_status st = ensure_scratch(gd, (directIn ? 0 : qf) + mf + n);
+        lf_status st = ensure_scratch(gd, (directIn ? 0 : qf) + (directMix ? 0 : mf) + n);
         if (st != LF_OK) return st;
     }
     float* next = staged ? reinterpret_cast<float*>(c->d_stage) : gd->scratch;
@@ -839,11 +842,11 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
             cudaMemcpyAsync(copy, queries, qf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
         dq = copy;
     }
-    float* const dmix = take(mf);
+    float* const dmix = directMix ? mix : take(mf);
     float* const dpdf = directPdf ? pdf : take((size_t)n);
     int ie;
     if (gd->tensorPath)
-        ie = launch_infer_tc(gd->net, dq, nullptr, n, dmix, c->d_status, c->stream, dpdf);
+        ie = launch_infer_tc(gd->net, dq, nullptr, n, dmix, c->d_status, c->stream, dpdf, directMix || staged);
     else
     {
         ie = launch_infer(gd->net, dq, nullptr, n, dmix, c->stream);
@@ -852,7 +855,7 @@ lf_status lf_guide_eval(lf_guide* gd, const float* queries, int32_t n, float* mi
     if (ie) return cuda_fail(c, (cudaError_t)ie, "guide inference launch");
     if (!staged)
     {
-        if (mix) cudaMemcpyAsync(mix, dmix, mf * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+        if (mix && !directMix) cudaMemcpyAsync(mix, dmix, mf * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
         if (pdf && !directPdf) cudaMemcpyAsync(pdf, dpdf, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
     }
     cudaError_t e = cudaStreamSynchronize(c->stream);

@@ -283,9 +283,9 @@ __device__ __forceinline__ float sample_loss_grad(const float* out, const float 
 int launch_infer(const Net& net, const float* queries, const int* nDev, int cap, float* mix, cudaStream_t st);
 // The same on the tcgen05 tensor cores (lf_guide_tc.cu): tiles of 128 queries, accumulators in
 // TMEM. A bounded wait that runs out sets LF_DEVERR_GUIDE_TIMEOUT in `status`. With `pdf` also the
-// density of each record's direction (floats 9..11).
+// density of each record's direction (floats 9..11). `lines`: mix is host memory, written by lines.
 int launch_infer_tc(const Net& net, const float* queries, const int* nDev, int cap, float* mix, uint32_t* status,
-                    cudaStream_t st, float* pdf = nullptr);
+                    cudaStream_t st, float* pdf = nullptr, bool lines = false);
 // One training pass on tcgen05 (lf_guide_tc.cu): the per-sample weight and grid gradients of n
 // sample records summed into gW / gGrid and the loss into `loss`, as the warp-level kernel.
 int launch_train_tc(const Net& net, const float* samples, int n, float* gW, float* gGrid, double* loss, uint32_t* status,
