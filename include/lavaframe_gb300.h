@@ -207,14 +207,17 @@ typedef struct lf_hit
 #define LF_TRACE_UNSORTED 0x4 /* trace in input order (large queries are binned by origin cell and octant) */
 #define LF_TRACE_SIMPLE 0x8   /* one thread per ray, no persistent warps */
 
-/* Host buffers: copies rays in, traces, copies hits out (synchronous). When the output lies
- * in one block from lf_host_alloc of this context, the kernels write the results there and
- * nothing is copied back. */
+/* Host buffers, synchronous. On a coherent host (the GPU walks the host's page tables) rays and
+ * results that are 16-byte aligned and do not overlap are read and written where they are, in
+ * input order (closest hits on scenes of more than 1.5M triangles from 2^19 rays up are
+ * binned instead). Otherwise: copies rays in, traces, copies hits out; when the output lies in one
+ * block from lf_host_alloc of this context, the kernels write the results there and nothing
+ * is copied back. */
 lf_status lf_trace_closest(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, lf_hit* hits, uint32_t flags);
 /* occluded[i] = 1 when something lies closer than tmax. */
 lf_status lf_trace_any(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, uint8_t* occluded, uint32_t flags);
 /* Host-buffer queries split the rays into `chunks` pieces (1..8; 0 = automatic, the
- * default: two pieces from 2^24 rays up, else one): piece k+1 is copied in and piece k-1
+ * default: two pieces from 2^24 rays up, else one; more than one always go over copies): piece k+1 is copied in and piece k-1
  * copied out while piece k is sorted and traced. Every ray's result is the same for any
  * setting; LF_TRACE_STATS queries run whole. */
 lf_status lf_ctx_set_host_chunks(lf_ctx* c, int32_t chunks);

@@ -728,7 +728,11 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     }
     cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);      // training steps leave theirs
     st = run_gradients(gd, in, n);
-    if (st != LF_OK) return st;
+    if (st != LF_OK)
+    {
+        cudaStreamSynchronize(c->stream);   // no kernel may still read the caller's samples
+        return st;
+    }
     guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(
         gd->wGrad, gd->gGrad, gd->dLoss, 1.f / (float)n, dW, outGrid, dW + kWeights);
     if (!directGrid) cudaMemcpyAsync(dgrid, outGrid, gridBytes, cudaMemcpyDeviceToHost, c->stream);
