@@ -92,8 +92,8 @@ int launch_trace_binned(const DevScene& S, const float4* rays, long long n, void
                         unsigned long long* next, uint32_t* status, cudaStream_t st, cudaEvent_t evStart = nullptr,
                         cudaEvent_t evStop = nullptr);
 int trace_bins();
-// Whether a query of n rays is binned unless its caller asks for input order.
-bool trace_sorts(long long n, bool any);
+// Whether a query of n rays against `tris` triangles is binned unless its caller asks for input order.
+bool trace_sorts(long long n, bool any, int tris);
 int launch_trace_any(const DevScene& S, const float4* rays, long long n, uint8_t* occ, int lights, bool stats,
                      uint32_t* status, unsigned long long* stat3, cudaStream_t st);
 }

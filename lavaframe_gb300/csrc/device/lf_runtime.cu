@@ -1108,7 +1108,7 @@ lf_status lf_trace_closest_device(lf_ctx* c, lf_scene* sc, const void* d_rays, i
     int e;
     if (!stats && !(flags & LF_TRACE_SIMPLE))
     {
-        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, false);
+        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, false, sc->view.trav.numTris);
         lf_status bs = ensure_bin_scratch(c, n, binned);
         if (bs != LF_OK) return bs;
         cudaEvent_t k0, k1;
@@ -1135,7 +1135,7 @@ lf_status lf_trace_any_device(lf_ctx* c, lf_scene* sc, const void* d_rays, int64
     int e;
     if (!stats && !(flags & LF_TRACE_SIMPLE))
     {
-        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, true);
+        const bool binned = !(flags & LF_TRACE_UNSORTED) && trace_sorts(n, true, sc->view.trav.numTris);
         lf_status bs = ensure_bin_scratch(c, n, binned);
         if (bs != LF_OK) return bs;
         cudaEvent_t k0, k1;
@@ -1196,9 +1196,10 @@ void read_trace_stats(lf_ctx* c)
 // 11.8 / 12.2 on 5.2M; equal on 10.5M. Sizes that are not binned either way: 8,000 closest hits 53 ->
 // 31 us, 300,000 179 -> 104.
 constexpr int kDirectClosestTris = 1500000;
+constexpr int64_t kDirectClosest = 1 << 19;   // and up to this many rays on any scene
 bool direct_query(const lf_scene* sc, int64_t n, bool any, uint32_t flags)
 {
-    return any || (flags & LF_TRACE_UNSORTED) || !trace_sorts(n, any) || sc->view.trav.numTris <= kDirectClosestTris;
+    return any || (flags & LF_TRACE_UNSORTED) || n < kDirectClosest || sc->view.trav.numTris <= kDirectClosestTris;
 }
 
 // Traces from and to the caller's buffers (direct_query), or copies the rays in, traces them and

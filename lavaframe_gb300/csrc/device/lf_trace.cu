@@ -28,14 +28,23 @@ constexpr int kScanBlocks = bins_of(kCellBits) / kScanBlock;   // partial sums o
 static_assert(kScanBlocks >= 1 && kScanBlocks <= 2 * kScanBlock, "bin scan covers 2^10 to 2^21 bins");
 
 // Sizes from which queries are binned. Binning costs about 20 us and two scattered passes; it pays
-// once many rays share a bin. Closest hit, binned / input order, us: 250k rays 496 / 545 on 1.3M
-// random triangles but 112 / 97, 170 / 131 and 85 / 64 on a room, spheres and the Cornell box; 1M
-// rays 1398 / 1583, 282 / 301, 385 / 383, 199 / 192; 4M rays 4971 / 5790, 941 / 1123, 1200 / 1303,
-// 626 / 709. Occlusion queries end early and write one byte per ray, which binning scatters: 4M
-// rays 4254 / 4460, 472 / 485, 1033 / 1048, 427 / 373; 16M rays 16.3 / 17.3, 1.89 / 1.87,
-// 3.96 / 3.86, 1.69 / 1.44 ms.
-// Queries of host buffers have a rule of their own (direct_query).
-constexpr long long kSortClosest = 1 << 19;
+// once many rays share a bin, the sooner the more the geometry's cache misses cost. Closest hits in
+// device memory, binned / input order, us. Up to 8k triangles (Cornell box, room, random): 2^20 rays
+// 151 / 139, 162 / 155, 148 / 121, 2^21 261 / 257, 285 / 287, 258 / 220, 2^22 on the Cornell box 456 / 492.
+// Up to 1.2M (Cornell 35k, room 48k, spheres 164k, random 327k): 524k rays 141 / 135, 169 / 175, 186 / 168,
+// 624 / 636, 800k 189 / 189, 230 / 245, 243 / 225, 889 / 907, 2^21 415 / 446, 517 / 585, 512 / 504,
+// 2148 / 2217: 2^19 lies between them (3 * 2^18 gives spheres 16 % there and takes 5 % from the
+// room). Beyond the L2 (1.3M, 2M, 5.2M random triangles): 131k 283 / 274, -, 407 / 401, 262k 445 / 492,
+// 495 / 534, 643 / 671, 524k 751 / 835, 779 / 935, 1047 / 1212. Queries of host buffers have a rule of
+// their own (direct_query).
+long long sort_closest(int tris)
+{
+    if (tris <= 1 << 13) return 1 << 21;
+    return tris <= 1200000 ? 1 << 19 : 1 << 18;
+}
+// Occlusion queries end early and write one byte per ray, which binning scatters: 4M rays on 1.3M random
+// triangles, a room, spheres and the Cornell box 4254 / 4460, 472 / 485, 1033 / 1048, 427 / 373; 16M
+// rays 16.3 / 17.3, 1.89 / 1.87, 3.96 / 3.86, 1.69 / 1.44 ms.
 constexpr long long kSortAny = 1 << 23;
 // 64^3 cells from here on, 32^3 below: 4M rays 4.94 / 4.97 ms on the random triangles, but 1.00 / 0.94,
 // 1.29 / 1.20 and 0.70 / 0.63 ms on the others; on 2^24 rays against 10.5M triangles 32^3 cells
@@ -350,7 +359,7 @@ int launch_trace_binned(const DevScene& S, const float4* rays, long long n, void
     return (int)cudaGetLastError();
 }
 
-bool trace_sorts(long long n, bool any) { return n >= (any ? kSortAny : kSortClosest); }
+bool trace_sorts(long long n, bool any, int tris) { return n >= (any ? kSortAny : sort_closest(tris)); }
 
 int trace_bins() { return bins_of(kCellBits) + kScanBlocks + 1; }   // counters, scan partial sums, block count
 }
