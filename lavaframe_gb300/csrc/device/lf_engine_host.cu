@@ -415,19 +415,31 @@ lf_status frame_render_fitting(lf_frame* f, EngineHost* e, const Params& Pf, int
                                                             f->numTilesY, f->accum, f->accum64, c->stream);
     if (le == 0 && tiles == 1)
     {
-        // the last pass stays readable (lf_frame_read_paths)
+        // the last pass stays readable (lf_frame_read_paths): of several a copy of it, or where there
+        // is no room for one the whole run's radiance - the samples are accumulated, so the
+        // call must not fail for it
         const EnginePass& last = run.back();
-        f->lastRadiance = arena;
-        f->lastRadianceSamples = last.nSamples;
+        float4* copy = nullptr;
         if (run.size() > 1)
         {
-            err = cudaMallocAsync((void**)&f->lastRadiance, sizeof(float4) * last.numPaths, c->stream);
-            if (err == cudaSuccess)
-                err = cudaMemcpyAsync(f->lastRadiance, last.radiance, sizeof(float4) * last.numPaths,
-                                      cudaMemcpyDeviceToDevice, c->stream);
-            cudaFreeAsync(arena, c->stream);
-            if (err != cudaSuccess) return cuda_fail(c, err, "pass radiance copy");
+            const size_t bytes = sizeof(float4) * (size_t)last.numPaths;
+            err = cudaMallocAsync((void**)&copy, bytes, c->stream);
+            if (err != cudaSuccess)
+            {
+                cudaGetLastError();
+                copy = nullptr;
+            }
+            else if ((err = cudaMemcpyAsync(copy, last.radiance, bytes, cudaMemcpyDeviceToDevice, c->stream)) != cudaSuccess)
+            {
+                cudaFreeAsync(copy, c->stream);
+                cudaFreeAsync(arena, c->stream);
+                return cuda_fail(c, err, "pass radiance copy");
+            }
         }
+        if (copy) cudaFreeAsync(arena, c->stream);
+        f->lastBlock = copy ? copy : arena;
+        f->lastRadiance = copy ? copy : last.radiance;
+        f->lastRadianceSamples = last.nSamples;
     }
     else
         cudaFreeAsync(arena, c->stream);
@@ -441,12 +453,7 @@ lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, in
     EngineHost* e = nullptr;
     lf_status st = engine_get(c, &e);
     if (st != LF_OK) return st;
-    if (f->lastRadiance)
-    {
-        cudaFreeAsync(f->lastRadiance, c->stream);
-        f->lastRadiance = nullptr;
-        f->lastRadianceSamples = 0;
-    }
+    drop_last_radiance(f);
     // a run whose paths fit the idle pool
     const long long paths = (long long)count * f->W * f->H;
     const long long passes = (long long)((count + f->sppBatch - 1) / f->sppBatch) * f->numTilesX * f->numTilesY;
@@ -483,7 +490,7 @@ lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, in
             const bool keep = i + 1 == run.size() && f->numTilesX * f->numTilesY == 1;
             if (keep)
             {
-                f->lastRadiance = q.radiance;
+                f->lastRadiance = f->lastBlock = q.radiance;
                 f->lastRadianceSamples = q.nSamples;
             }
             else

@@ -122,9 +122,10 @@ struct lf_frame
     cudaGraphExec_t graph = nullptr;
     int graphDepth = -1;
     // engine path (default): job slot in the context's engine and the per-path radiance of
-    // the most recent pass ([sample][pixel] of a single-tile frame)
+    // the most recent pass ([sample][pixel] of a single-tile frame), in the allocation lastBlock
     int engineJob = -1;
     float4* lastRadiance = nullptr;
+    float4* lastBlock = nullptr;
     int lastRadianceSamples = 0;
     // learned path guiding (per-batch pipeline, one sample per batch)
     lf_guide* guide = nullptr;
@@ -182,6 +183,14 @@ inline lf_status check_device(lf_ctx* c)
         return fail(c, LF_ERR_DEVICE, "device error bits 0x" + std::to_string(bits));
     }
     return LF_OK;
+}
+
+// Lets go of the most recent pass's radiance (in stream order).
+inline void drop_last_radiance(lf_frame* f)
+{
+    if (f->lastBlock) cudaFreeAsync(f->lastBlock, f->ctx->stream);
+    f->lastRadiance = f->lastBlock = nullptr;
+    f->lastRadianceSamples = 0;
 }
 
 // Kernel parameters of one render (lf_render_params + scene facts); tile fields cover the

@@ -1647,12 +1647,7 @@ lf_status frame_render_guided(lf_frame* f, Params P, int firstSample, int count)
         lf_status st = alloc_guide_buffers(f, cap);
         if (st != LF_OK) return st;
     }
-    if (f->lastRadiance)
-    {
-        cudaFreeAsync(f->lastRadiance, c->stream);
-        f->lastRadiance = nullptr;
-        f->lastRadianceSamples = 0;
-    }
+    drop_last_radiance(f);
     const bool tiledFrames = (f->flags & LF_FRAME_TILED_FRAMES) != 0;
     for (int s = 0; s < count;)
     {
@@ -1715,12 +1710,7 @@ lf_status lf_frame_render(lf_frame* f, int32_t first_sample, int32_t count)
         if (st == LF_OK) f->paths += (uint64_t)count * f->W * f->H;
         return st;
     }
-    if (f->lastRadiance)
-    {
-        cudaFreeAsync(f->lastRadiance, c->stream);
-        f->lastRadiance = nullptr;
-        f->lastRadianceSamples = 0;
-    }
+    drop_last_radiance(f);
     int s = 0;
     while (s < count)
     {
@@ -1753,12 +1743,7 @@ lf_status lf_frame_render_tile(lf_frame* f, int32_t sample, int32_t tile_x, int3
     P.tileX = tile_x;
     P.tileY = tile_y;
     P.tileOrdinal = tiledFrames ? (f->numTilesY - 1 - tile_y) * f->numTilesX + tile_x : 0;
-    if (f->lastRadiance)
-    {
-        cudaFreeAsync(f->lastRadiance, c->stream);
-        f->lastRadiance = nullptr;
-        f->lastRadianceSamples = 0;
-    }
+    drop_last_radiance(f);
     lf_status st = run_batch(f, P, sample, 1);
     if (st == LF_OK) f->paths += (uint64_t)f->P.tileW * f->P.tileH;
     return st;
@@ -1894,9 +1879,9 @@ lf_status lf_frame_release(lf_frame* f)
     if (!f) return LF_ERR_INVALID;
     cudaSetDevice(f->ctx->device);
     cudaStreamSynchronize(f->ctx->stream);
-    if (f->lastRadiance)
+    if (f->lastBlock)
     {
-        cudaFreeAsync(f->lastRadiance, f->ctx->stream);
+        drop_last_radiance(f);
         cudaStreamSynchronize(f->ctx->stream);
     }
     if (f->engineJob >= 0 && f->ctx->engine) engine_job_free(f->ctx->engine, f->engineJob);

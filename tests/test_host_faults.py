@@ -1,0 +1,28 @@
+"""Host code of the library when allocations or launches fail and while copies are still waiting, on
+a CUDA runtime in host memory (tests/fake_cuda.cpp)."""
+import lavaframe_gb300 as lf
+from tests.fakecuda import fake, fake_lib  # noqa: F401 (fixtures)
+
+
+def _frame(ctx, width=16, height=8, batch=2):
+    scene = ctx.upload(lf.HostScene().gen_cornell(width, height).build())
+    p = lf.HostScene().gen_cornell(width, height).build().render_params()
+    f = lf.Frame(ctx, scene, p)
+    f.set_batch(batch)
+    return scene, f
+
+
+def test_no_room_for_the_last_pass(fake):  # noqa: F811
+    """A run of several passes keeps the last one's radiance: without memory for a copy of it the frame
+    holds on to the whole run's, and frees it once."""
+    with lf.Context(0) as ctx:
+        scene, f = _frame(ctx)
+        f.render(0, 5)            # makes the engine
+        fake.fake_fail_alloc(1)   # after the run's radiance
+        f.render(5, 5)
+        assert f.paths(1).shape[1:] == (8, 16, 3)
+        f.render(10, 5)
+        assert fake.fake_block(16 * 8 * 16, 1)
+        f.close()
+        assert fake.fake_bad_frees() == 0 and fake.fake_pool_blocks(0) == 0
+        scene.close()
