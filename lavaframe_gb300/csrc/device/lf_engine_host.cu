@@ -87,6 +87,8 @@ lf_status engine_get(lf_ctx* c, EngineHost** out)
     A(&e->runPasses, kPassRing);
     if (err == cudaSuccess) err = cudaMallocHost((void**)&e->h_jobStage, sizeof(EngineJob) * kMaxJobs);
     if (err == cudaSuccess) err = cudaMallocHost((void**)&e->h_passStage, sizeof(EnginePass) * kPassRing);
+    if (err == cudaSuccess) err = cudaMallocHost((void**)&e->h_runStage, sizeof(EnginePass) * kPassRing);
+    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e->runCopied, cudaEventDisableTiming);
     for (int k = 0; k < 2 && err == cudaSuccess; ++k)
     {
         err = cudaMallocHost((void**)&e->h_ctl[k], sizeof(EngineCtl));
@@ -128,6 +130,8 @@ void engine_destroy(EngineHost* e)
     for (void* p : e->tables) cudaFree(p);
     if (e->h_jobStage) cudaFreeHost(e->h_jobStage);
     if (e->h_passStage) cudaFreeHost(e->h_passStage);
+    if (e->h_runStage) cudaFreeHost(e->h_runStage);
+    if (e->runCopied) cudaEventDestroy(e->runCopied);
     for (int k = 0; k < 2; ++k)
     {
         if (e->h_ctl[k]) cudaFreeHost(e->h_ctl[k]);
@@ -382,7 +386,16 @@ lf_status frame_render_fitting(lf_frame* f, EngineHost* e, const Params& Pf, int
     }
     if (run.size() > 1)
     {
-        err = cudaMemcpyAsync(e->runPasses, run.data(), sizeof(EnginePass) * run.size(), cudaMemcpyHostToDevice, c->stream);
+        // the call returns before the copy has run: it reads page-locked memory, and the next run of
+        // several passes waits for it before it writes there (an event that was never recorded has passed)
+        const size_t bytes = sizeof(EnginePass) * run.size();
+        err = cudaEventSynchronize(e->runCopied);
+        if (err == cudaSuccess)
+        {
+            std::memcpy(e->h_runStage, run.data(), bytes);
+            err = cudaMemcpyAsync(e->runPasses, e->h_runStage, bytes, cudaMemcpyHostToDevice, c->stream);
+        }
+        if (err == cudaSuccess) err = cudaEventRecord(e->runCopied, c->stream);
         if (err != cudaSuccess)
         {
             cudaFreeAsync(arena, c->stream);

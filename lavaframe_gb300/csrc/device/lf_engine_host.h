@@ -15,6 +15,8 @@ struct EngineHost
     size_t poolBytes = 0;
     unsigned long long* ownCtr = nullptr;   // counters of runs not tied to a frame
     EnginePass* runPasses = nullptr;        // pass table of the runs on the idle pool
+    EnginePass* h_runStage = nullptr;       // pinned staging of that table, written again after runCopied
+    cudaEvent_t runCopied = nullptr;
     EngineJob* h_jobStage = nullptr;        // pinned staging of the job table
     EnginePass* h_passStage = nullptr;      // pinned staging of the pass ring
     EngineCtl* h_ctl[2] = {nullptr, nullptr};

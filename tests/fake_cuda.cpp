@@ -21,6 +21,7 @@ struct Op
     size_t bytes;
     int value;
     bool pageable;   // a copy from host memory that is not page-locked
+    size_t sum;      // of a copy to the device: its source when it was asked for
 };
 struct Block
 {
@@ -34,7 +35,7 @@ std::deque<Op> queue;
 std::map<char*, Block> blocks;
 std::map<const void*, std::string> kernels;
 std::map<const void*, std::pair<void*, size_t>> vars;
-int badFrees = 0, failAlloc = -1, failLaunch = -1, badPoolUse = 0, coherent = 0;
+int badFrees = 0, changedSources = 0, failAlloc = -1, failLaunch = -1, coherent = 0;
 cudaError_t lastError = cudaSuccess;
 int defaultPool, defaultPoolChanges = 0, pools = 0;
 void (*hook)(const char*) = nullptr;
@@ -52,12 +53,20 @@ std::map<char*, Block>::iterator holding(const void* p)
     return (char*)p < it->first + it->second.bytes ? it : blocks.end();
 }
 
+size_t checksum(const void* p, size_t n)
+{
+    size_t h = 1469598103934665603ull;
+    for (size_t i = 0; i < n; ++i) h = (h ^ ((const unsigned char*)p)[i]) * 1099511628211ull;
+    return h;
+}
+
 void flush()
 {
     while (!queue.empty())
     {
         const Op o = queue.front();
         queue.pop_front();
+        if (o.sum && o.sum != checksum(o.src, o.bytes)) ++changedSources;
         if (o.kind == 0) std::memmove(o.dst, o.src, o.bytes);
         if (o.kind == 1) std::memset(o.dst, o.value, o.bytes);
         if (o.kind == 2) std::free(o.dst);
@@ -90,7 +99,7 @@ cudaError_t release(void* p, int kind)
         return done(cudaErrorInvalidValue);
     }
     blocks.erase(it);
-    queue.push_back({2, p, nullptr, 0, 0, false});
+    queue.push_back({2, p, nullptr, 0, 0, false, 0});
     if (kind != 1) flush();
     return cudaSuccess;
 }
@@ -110,17 +119,27 @@ void fake_reset()
 {
     Lock l(mu);
     flush();
-    badFrees = defaultPoolChanges = badPoolUse = 0;
+    badFrees = changedSources = defaultPoolChanges = 0;
     failAlloc = failLaunch = -1;
     lastError = cudaSuccess;
     hook = nullptr;
     coherent = 0;
+}
+void fake_flush()
+{
+    Lock l(mu);
+    flush();
 }
 void fake_fail_alloc(int after) { failAlloc = after; }     // the allocation that `after` others precede
 void fake_fail_launch(int after) { failLaunch = after; }
 void fake_hook(void (*f)(const char*)) { hook = f; }       // called for every launch with the kernel's name
 void fake_coherent(int on) { coherent = on; }
 int fake_bad_frees() { return badFrees; }
+int fake_changed_sources()   // copies whose source was written between the call and the copy
+{
+    fake_flush();
+    return changedSources;
+}
 int fake_pending() { return (int)queue.size(); }
 int fake_pending_pageable()
 {
@@ -128,11 +147,6 @@ int fake_pending_pageable()
     int n = 0;
     for (const Op& o : queue) n += o.kind == 0 && o.pageable;
     return n;
-}
-void fake_flush()
-{
-    Lock l(mu);
-    flush();
 }
 int fake_default_pool_changes() { return defaultPoolChanges; }
 int fake_pools() { return pools; }
@@ -168,7 +182,8 @@ cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned)
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t)
 {
     Lock l(mu);
-    queue.push_back({0, d, s, n, 0, k == cudaMemcpyHostToDevice && holding(s) == blocks.end()});
+    const bool in = k == cudaMemcpyHostToDevice;
+    queue.push_back({0, d, s, n, 0, in && holding(s) == blocks.end(), in ? checksum(s, n) : 0});
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind)
@@ -181,7 +196,7 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind)
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t)
 {
     Lock l(mu);
-    queue.push_back({1, d, nullptr, n, v, false});
+    queue.push_back({1, d, nullptr, n, v, false, 0});
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void* d, int v, size_t n)

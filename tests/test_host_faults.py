@@ -26,3 +26,16 @@ def test_no_room_for_the_last_pass(fake):  # noqa: F811
         f.close()
         assert fake.fake_bad_frees() == 0 and fake.fake_pool_blocks(0) == 0
         scene.close()
+
+
+def test_no_copy_from_memory_that_is_gone(fake):  # noqa: F811
+    """A render of several passes returns before its work has run: what its copies still have to read is
+    page-locked memory of the engine, which is written again only after they have."""
+    with lf.Context(0) as ctx:
+        scene, f = _frame(ctx)
+        f.render(0, 5)
+        assert fake.fake_pending() > 0 and fake.fake_pending_pageable() == 0
+        f.render(5, 5)
+        assert fake.fake_changed_sources() == 0
+        f.close()
+        scene.close()
