@@ -749,7 +749,18 @@ lf_status lf_guide_train_device(lf_guide* gd, const float* d_samples, int32_t n,
     lf_ctx* c = gd->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    lf_status st = run_gradients(gd, d_samples, n);
+    lf_status st = LF_OK;
+    if (gd->tensorPath && reinterpret_cast<uintptr_t>(d_samples) % 16)
+    {
+        // the tcgen05 kernel loads 16 bytes at a time: records that start elsewhere are moved first
+        const size_t floats = (size_t)n * kSampleFloats;
+        st = ensure_scratch(gd, floats);
+        if (st != LF_OK) return st;
+        const cudaError_t ce = cudaMemcpyAsync(gd->scratch, d_samples, floats * sizeof(float), cudaMemcpyDeviceToDevice, c->stream);
+        if (ce != cudaSuccess) return cuda_fail(c, ce, "guide samples");
+        d_samples = gd->scratch;
+    }
+    st = run_gradients(gd, d_samples, n);
     if (st != LF_OK) return st;
     ++gd->step;
     const float b1 = 0.9f, b2 = 0.99f, eps = 1e-8f;

@@ -38,7 +38,7 @@ std::map<const void*, std::pair<void*, size_t>> vars;
 int badFrees = 0, changedSources = 0, failAlloc = -1, failLaunch = -1, coherent = 0;
 cudaError_t lastError = cudaSuccess;
 int defaultPool, defaultPoolChanges = 0, pools = 0;
-void (*hook)(const char*) = nullptr;
+void (*hook)(const char*, void**) = nullptr;
 dim3 cfgGrid, cfgBlock;
 size_t cfgSmem;
 cudaStream_t cfgStream;
@@ -104,11 +104,11 @@ cudaError_t release(void* p, int kind)
     return cudaSuccess;
 }
 
-cudaError_t launch(const void* f)
+cudaError_t launch(const void* f, void** args)
 {
     Lock l(mu);
     if (failLaunch >= 0 && failLaunch-- == 0) return done(cudaErrorLaunchOutOfResources);
-    if (hook) hook(kernels[f].c_str());
+    if (hook) hook(kernels[f].c_str(), args);
     return cudaSuccess;
 }
 }
@@ -132,7 +132,8 @@ void fake_flush()
 }
 void fake_fail_alloc(int after) { failAlloc = after; }     // the allocation that `after` others precede
 void fake_fail_launch(int after) { failLaunch = after; }
-void fake_hook(void (*f)(const char*)) { hook = f; }       // called for every launch with the kernel's name
+// called for every launch with the kernel's name and the addresses of its arguments
+void fake_hook(void (*f)(const char*, void**)) { hook = f; }
 void fake_coherent(int on) { coherent = on; }
 int fake_bad_frees() { return badFrees; }
 int fake_changed_sources()   // copies whose source was written between the call and the copy
@@ -324,7 +325,7 @@ cudaError_t cudaGetSymbolAddress(void** p, const void* symbol)
     *p = vars[symbol].first;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void**) { return launch(f); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launch(f, args); }
 
 // what the compiler's host stubs call
 unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t m, cudaStream_t s)
@@ -348,7 +349,10 @@ cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* f)
     *k = (cudaKernel_t)f;
     return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t, cudaStream_t) { return launch((const void*)k); }
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** args, size_t, cudaStream_t)
+{
+    return launch((const void*)k, args);
+}
 void** __cudaRegisterFatBinary(void*)
 {
     static void* h;

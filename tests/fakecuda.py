@@ -10,7 +10,7 @@ import lavaframe_gb300 as lf
 from lavaframe_gb300 import build
 from tests.conftest import ROOT
 
-HOOK = C.CFUNCTYPE(None, C.c_char_p)
+HOOK = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.POINTER(C.c_void_p)))
 POOL, PINNED = 1, 2
 
 

@@ -1,7 +1,12 @@
 """Host code of the library when allocations or launches fail and while copies are still waiting, on
 a CUDA runtime in host memory (tests/fake_cuda.cpp)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
 import lavaframe_gb300 as lf
-from tests.fakecuda import fake, fake_lib  # noqa: F401 (fixtures)
+from tests.fakecuda import HOOK, fake, fake_lib  # noqa: F401 (fixtures)
 
 
 def _frame(ctx, width=16, height=8, batch=2):
@@ -39,3 +44,29 @@ def test_no_copy_from_memory_that_is_gone(fake):  # noqa: F811
         assert fake.fake_changed_sources() == 0
         f.close()
         scene.close()
+
+
+@pytest.mark.parametrize("by", [0, 4, 8, 12, 16])
+def test_device_samples_reach_the_kernel_aligned(fake, by):  # noqa: F811
+    """The tcgen05 training kernel loads its records 16 bytes at a time; a device pointer may be aligned
+    for floats only."""
+    n, seen = 200, []
+    want = np.arange(n * 16, dtype=np.float32)
+
+    def launched(name, args):
+        if b"guide_train_tc_kernel" in name:
+            fake.fake_flush()
+            seen.append((args[1][0] % 16, bytes((C.c_char * want.nbytes).from_address(args[1][0])) == want.tobytes()))
+
+    with lf.Context(0) as ctx:
+        g = lf.Guide(ctx, [0, 0, 0], [1, 1, 1], seed=3)
+        d = C.c_void_p()
+        ctx._c(fake.lf_device_alloc(ctx.h, want.nbytes + 16, C.byref(d)))
+        C.memmove(d.value + by, want.ctypes.data, want.nbytes)
+        hook = HOOK(launched)
+        fake.fake_hook(hook)
+        ctx._c(fake.lf_guide_train_device(g.h, C.c_void_p(d.value + by), n, 1e-2))
+        fake.fake_hook(HOOK())
+        assert seen == [(0, True)]
+        ctx._c(fake.lf_device_free(ctx.h, d))
+        g.close()
