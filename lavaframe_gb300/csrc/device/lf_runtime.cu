@@ -325,8 +325,8 @@ lf_status encode_level(lf_ctx* c, const RefNode* nodes, int numNodes, int start,
 // binary encoding's codes (instances with kWideInstLeaf set); every child slot carries the
 // reference node's own box and index.
 //
-// An instance whose inverse transform is the identity and whose mesh no other instance uses is
-// merged into the instance level: its leaf counts as the mesh's root, so nodes may collapse
+// An instance whose inverse transform is the identity and whose mesh no other instance uses, not even
+// in parts (mark_shared), is merged into the instance level: its leaf counts as the mesh's root, so nodes may collapse
 // across the two levels and its triangles are leaves of the instance level's tree. The object
 // ray of such an instance is the world ray (the transform's products and sums reproduce every
 // finite component, and a zero origin component as +0), so the boxes and triangles tested give
@@ -397,6 +397,43 @@ bool inlinable(const WideBuilder& B, int leaf, int root)
             if (!(C.bmin[a] >= L.bmin[a] && C.bmax[a] <= L.bmax[a])) return false;
     }
     return true;
+}
+
+// Marks in `shared` (by root) the meshes that have a reference node or a triangle in common with
+// another mesh. Only the others may be merged: a merged mesh's nodes are taken up by the instance
+// level and its triangles carry its instance.
+void mark_shared(const WideBuilder& B, const std::vector<int>& roots, std::vector<unsigned char>& shared)
+{
+    std::vector<int> nodeOwner(B.numNodes, -1), triOwner(B.numTris, -1), stack;
+    auto meets = [&](int root, int other) {
+        if (other >= 0 && other != root) shared[root] = shared[other] = 1;
+        return other >= 0;
+    };
+    for (const int root : roots)
+    {
+        if (root < 0 || root >= B.numNodes || nodeOwner[root] == root) continue;
+        stack.push_back(root);
+        while (!stack.empty())
+        {
+            const int k = stack.back();
+            stack.pop_back();
+            if (meets(root, nodeOwner[k])) continue;   // what lies below is the other mesh's already
+            nodeOwner[k] = root;
+            const RefNode& n = B.nodes[k];
+            const int l = (int)n.lr[0], r = (int)n.lr[1];
+            if ((int)n.lr[2] == 0)
+            {
+                stack.push_back(r);
+                stack.push_back(l);
+            }
+            else
+                for (int t = l; t < l + r; ++t)
+                {
+                    meets(root, triOwner[t]);
+                    triOwner[t] = root;
+                }
+        }
+    }
 }
 
 float box_area(const RefNode& n)
@@ -544,10 +581,12 @@ lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, s
         }
     }
     // instances merged into the instance level: identity inverse (bit for bit), a mesh of their own
+    std::vector<unsigned char> shared(v->num_nodes, 0);
+    mark_shared(B, instRoot, shared);
     const float4 identity[3] = {make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0)};
     for (int i = 0; i < v->num_instances; ++i)
         if (instRoot[i] >= 0 && instRoot[i] < v->num_nodes && rootUses[instRoot[i]] == 1 &&
-            std::memcmp(&inst[(size_t)i * 4], identity, sizeof identity) == 0 && inlinable(B, instLeaf[i], instRoot[i]))
+            !shared[instRoot[i]] && std::memcmp(&inst[(size_t)i * 4], identity, sizeof identity) == 0 && inlinable(B, instLeaf[i], instRoot[i]))
             B.inlineRoot[i] = instRoot[i];
     for (int i = 0; i < v->num_instances; ++i)
     {

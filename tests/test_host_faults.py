@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import lavaframe_gb300 as lf
+from tests import shared_meshes
 from tests.fakecuda import HOOK, fake, fake_lib  # noqa: F401 (fixtures)
 
 
@@ -70,3 +71,10 @@ def test_device_samples_reach_the_kernel_aligned(fake, by):  # noqa: F811
         assert seen == [(0, True)]
         ctx._c(fake.lf_device_free(ctx.h, d))
         g.close()
+
+
+@pytest.mark.parametrize("kind", shared_meshes.KINDS)
+def test_meshes_that_share_nodes_are_accepted(fake, kind):  # noqa: F811
+    """A mesh may be a part of another one's tree."""
+    with lf.Context(0) as ctx:
+        shared_meshes.upload(ctx, shared_meshes.View(kind)).close()
