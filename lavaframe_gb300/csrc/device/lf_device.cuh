@@ -65,7 +65,11 @@ constexpr int kWide = LF_WIDE;
 static_assert(kWide == 4 || kWide == 8, "wide nodes have 4 or 8 children");
 constexpr int kWideF4 = 2 * kWide;
 constexpr int kWideEmpty = (int)0x80000002;
-constexpr int kWideInstLeaf = 1 << 28;   // leaf payload bit: an instance (else a run of triangles)
+// Leaf payloads (the complement of a leaf's code): an instance with this bit, else a run of triangles,
+// 4 * first + count. Scenes of more than kWideTris triangles, whose runs would reach the bit, keep
+// the binary traversal.
+constexpr int kWideInstLeaf = 1 << 30;
+constexpr int kWideTris = kWideInstLeaf >> 2;
 constexpr int kWideStack = kWide == 8 ? 160 : 96;
 
 struct DevScene

@@ -894,7 +894,7 @@ lf_status lf_scene_upload(lf_ctx* c, const lf_scene_view* v, lf_scene** out)
     S.trav.numInstances = v->num_instances;
     S.trav.cullRel = 1.0e-4f;
     S.trav.cullAbs = 64.0f * ulp_of(extent);
-    S.trav.wnodes = d_wide;
+    S.trav.wnodes = v->num_tris <= kWideTris ? d_wide : nullptr;
     S.trav.wroot = wroot;
     S.trav.wideOn = 1;
     S.trav.refNodes = d_refNodes;
@@ -987,7 +987,7 @@ lf_status lf_scene_update_instances(lf_scene* sc, const lf_scene_view* v)
             sc->bytes += (wideNodes - sc->wideCapacity) * kWideF4 * sizeof(float4);
             sc->wideCapacity = wideNodes;
             sc->d_wide = grown;
-            sc->view.trav.wnodes = grown;
+            if (sc->view.trav.wnodes) sc->view.trav.wnodes = grown;
         }
     }
     if (e == cudaSuccess)
