@@ -2083,9 +2083,21 @@ extern "C" lf_status lf_render_noalloc(lf_scene* sc, const lf_render_params* p, 
     b.cap = (int)N;
     b.shadeThreadsPerSm = kDefaultShadeCap;
 
+    // Ends the call, also one whose launch failed: earlier passes may still run, and the status word is this
+    // call's alone.
+    auto finish = [&](cudaError_t err, const char* what) {
+        const cudaError_t sync = cudaStreamSynchronize(c->stream);
+        const uint32_t bits = c->h_status[1];
+        c->h_status[1] = 0;
+        c->devErrors |= bits;
+        if (err != cudaSuccess) return cuda_fail(c, err, what);
+        if (sync != cudaSuccess) return cuda_fail(c, sync, "no-alloc render");
+        return bits ? fail(c, LF_ERR_DEVICE, "device error bits 0x" + std::to_string(bits)) : LF_OK;
+    };
+
     // the array keeps the previous call's contents: clear the counters
     cudaError_t e = cudaMemsetAsync(base, 0, kNoAllocHeader, c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "no-alloc scratch clear");
+    if (e != cudaSuccess) return finish(e, "no-alloc scratch clear");
 
     EngineJob one;
     std::memset(&one, 0, sizeof one);
@@ -2112,18 +2124,9 @@ extern "C" lf_status lf_render_noalloc(lf_scene* sc, const lf_render_params* p, 
                 int le = launch_frame_run(b, one, q, table, 1, (int)q.numPaths, radiance,
                                           std::numeric_limits<int>::max(), c->stream);
                 if (le == 0) le = launch_engine_accumulate(P, q, (float4*)d_accum, nullptr, c->stream);
-                if (le) return cuda_fail(c, (cudaError_t)le, "no-alloc render launch");
+                if (le) return finish((cudaError_t)le, "no-alloc render launch");
             }
         s += n;
     }
-    e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return cuda_fail(c, e, "no-alloc render");
-    const uint32_t bits = c->h_status[1];
-    c->h_status[1] = 0;
-    if (bits)
-    {
-        c->devErrors |= bits;
-        return fail(c, LF_ERR_DEVICE, "device error bits 0x" + std::to_string(bits));
-    }
-    return LF_OK;
+    return finish(cudaSuccess, "no-alloc render");
 }

@@ -7,7 +7,7 @@ import pytest
 
 import lavaframe_gb300 as lf
 from tests import shared_meshes
-from tests.fakecuda import HOOK, fake, fake_lib  # noqa: F401 (fixtures)
+from tests.fakecuda import HOOK, PINNED, fake, fake_lib  # noqa: F401 (fixtures)
 
 
 def _frame(ctx, width=16, height=8, batch=2):
@@ -78,3 +78,32 @@ def test_meshes_that_share_nodes_are_accepted(fake, kind):  # noqa: F811
     """A mesh may be a part of another one's tree."""
     with lf.Context(0) as ctx:
         shared_meshes.upload(ctx, shared_meshes.View(kind)).close()
+
+
+def test_noalloc_reports_its_own_errors(fake):  # noqa: F811
+    """A render without allocation whose launch fails returns once its earlier passes are done, and their
+    error bits are not the next call's."""
+    p = lf.HostScene().gen_cornell(64, 32).build().render_params()
+    p.tile_width, p.tile_height = 32, 32
+    with lf.Context(0) as ctx:
+        scene = ctx.upload(lf.HostScene().gen_cornell(64, 32).build())
+        d = C.c_void_p()
+        ctx._c(fake.lf_device_alloc(ctx.h, 64 * 32 * 16, C.byref(d)))
+        status = C.cast(fake.fake_block(8, PINNED), C.POINTER(C.c_uint32))
+
+        def launched(name, args):
+            if b"engine_direct_kernel" in name:
+                status[1] = 1
+
+        hook = HOOK(launched)
+        fake.fake_hook(hook)
+        assert fake.lf_render_noalloc(scene.h, C.byref(p), 0, 1, d) == 4   # the bit is reported
+        assert fake.lf_render_noalloc(scene.h, C.byref(p), 0, 1, d) == 4 and status[1] == 0
+        fake.fake_fail_launch(2)   # the second tile's first kernel
+        assert fake.lf_render_noalloc(scene.h, C.byref(p), 0, 1, d) == 2
+        assert fake.fake_pending() == 0
+        fake.fake_hook(HOOK())
+        assert fake.lf_render_noalloc(scene.h, C.byref(p), 0, 1, d) == 0
+        assert ctx.device_errors() == 1
+        ctx._c(fake.lf_device_free(ctx.h, d))
+        scene.close()
