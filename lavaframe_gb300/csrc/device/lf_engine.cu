@@ -689,13 +689,13 @@ __global__ void __maxnreg__(64) engine_shadow_kernel(EngineBuffers b, EngineJob 
 constexpr int kRunBlock = 256;
 
 // Takes the path in slot p (-1: none) of every thread of the block from its extension ray to its end;
-// adds up the extension and shadow rays. `job()` gives the scene and parameters of the thread's path.
+// adds up the extension and shadow rays. Its depth is at most kThreadBounces. `job()` gives the scene and parameters of the thread's path.
 template <bool kLights, class Job>
 __device__ __forceinline__ void run_paths(const PathSoA& ps, uint32_t* status, unsigned long long* ctr, int p, Job job,
                                           unsigned long long& ext, unsigned long long& shadowRays)
 {
     bool alive = p >= 0;
-    for (int bounce = 0; bounce < 4096 && __syncthreads_or(alive); ++bounce)
+    for (int bounce = 0; bounce < kThreadBounces && __syncthreads_or(alive); ++bounce)
     {
         if (alive)
         {
@@ -1045,7 +1045,8 @@ int launch_frame_run(const EngineBuffers& b0, const EngineJob& one, const Engine
 {
     EngineBuffers b = b0;
     b.passes = table;
-    if (one.P.maxDepth <= 0 || n <= std::min(kDirectPaths, drainPaths))
+    const bool deep = one.P.maxDepth > kThreadBounces;
+    if (one.P.maxDepth <= 0 || (!deep && n <= std::min(kDirectPaths, drainPaths)))
     {
         b.ps.L = radiance;
         auto direct = [&](auto kernel) {
@@ -1057,10 +1058,10 @@ int launch_frame_run(const EngineBuffers& b0, const EngineJob& one, const Engine
     }
     launch_chained(engine_start_kernel, full_grid((const void*)engine_start_kernel, 256, n), 256, st, b, one.P, first, table,
                    numPasses, n);
-    const int bounces = std::min(one.P.maxDepth, kRunBounces);
+    const int bounces = deep ? one.P.maxDepth : std::min(one.P.maxDepth, kRunBounces);
     for (int k = 0; k < bounces; ++k)
     {
-        if ((k == 2 || k == 4) && bounces - k > 1) drain<true>(b, one, k & 1, n, std::min(kDrainPaths, drainPaths), st);
+        if (!deep && (k == 2 || k == 4) && bounces - k > 1) drain<true>(b, one, k & 1, n, std::min(kDrainPaths, drainPaths), st);
         bounce<true>(b, one, k & 1, n, st);
     }
     if (bounces < one.P.maxDepth) drain<true>(b, one, bounces & 1, n, n, st);

@@ -36,6 +36,7 @@ namespace lfd
 constexpr int kPassRingBits = 14;
 constexpr int kPassRing = 1 << kPassRingBits;   // pass descriptors in flight
 constexpr int kMaxEngineJobs = 1 << 16;         // job slots (packed into the upper bits of info.w)
+constexpr int kThreadBounces = 4096;            // most bounces that one thread takes a path through in one launch
 constexpr int kDefaultShadeCap = 512;           // shade kernel register cap (threads per SM)
 
 struct EngineJob
@@ -106,7 +107,8 @@ int launch_engine_drain(const EngineBuffers& b, const EngineJob* one, cudaStream
 // (= b.passes; `first` is written there when the run has one pass), whose pathBase counts from 0 in
 // increasing order and whose radiance lies at radiance + pathBase. Small runs are traced by one
 // launch, larger ones by one launch per kernel and bounce. drainPaths bounds the paths that one thread each
-// takes to their ends.
+// takes to their ends; no thread does for depths above kThreadBounces, so that no launch runs for as long
+// as a caller's depth likes: those runs launch every bounce.
 int launch_frame_run(const EngineBuffers& b, const EngineJob& one, const EnginePass& first, EnginePass* table,
                      int numPasses, int n, float4* radiance, int drainPaths, cudaStream_t st);
 // Per-pixel sums of a run's passes - chunks of samples, each with every tile in TiledRenderer's

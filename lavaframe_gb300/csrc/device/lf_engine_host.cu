@@ -339,7 +339,7 @@ lf_status engine_drain(EngineHost* e, unsigned long long* ctr, int maxDepth, int
         const EngineCtl& s = *e->h_ctl[cur];
         if (s.active == 0 && s.next >= s.total) break;
         // once every id is issued and few paths remain, run them to their ends in one kernel
-        if (e->drainPaths > 0 && s.next >= s.total && s.active <= e->drainPaths) drain = true;
+        if (e->drainPaths > 0 && maxDepth <= kThreadBounces && s.next >= s.total && s.active <= e->drainPaths) drain = true;
         if (++pairs * 2 > limit) return fail(c, LF_ERR_DEVICE, "engine did not drain");
         cur ^= 1;
     }
@@ -467,10 +467,10 @@ lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, in
     lf_status st = engine_get(c, &e);
     if (st != LF_OK) return st;
     drop_last_radiance(f);
-    // a run whose paths fit the idle pool
+    // a run whose paths fit the idle pool (deeper ones are looked at while they run, to end with their last path)
     const long long paths = (long long)count * f->W * f->H;
     const long long passes = (long long)((count + f->sppBatch - 1) / f->sppBatch) * f->numTilesX * f->numTilesY;
-    if (e->active == 0 && e->drainPaths > 0 && passes <= kPassRing && paths <= e->b.cap &&
+    if (e->active == 0 && e->drainPaths > 0 && Pf.maxDepth <= kThreadBounces && passes <= kPassRing && paths <= e->b.cap &&
         (size_t)paths * sizeof(float4) <= kRunRadianceBytes)
         return frame_render_fitting(f, e, Pf, firstSample, count, paths);
     if (f->engineJob < 0)
