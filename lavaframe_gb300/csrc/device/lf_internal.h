@@ -153,6 +153,7 @@ inline lf_status fail(lf_ctx* c, lf_status st, const std::string& msg)
 inline lf_status cuda_fail(lf_ctx* c, cudaError_t e, const char* what)
 {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();   // reported here: the next launch's check must not find it again
     if (e == cudaErrorMemoryAllocation) return fail(c, LF_ERR_OOM, m);
     return fail(c, LF_ERR_CUDA, m);
 }

@@ -7,7 +7,7 @@ import pytest
 
 import lavaframe_gb300 as lf
 from tests import shared_meshes
-from tests.fakecuda import HOOK, PINNED, fake, fake_lib  # noqa: F401 (fixtures)
+from tests.fakecuda import HOOK, PINNED, POOL, fake, fake_lib  # noqa: F401 (fixtures)
 
 
 def _frame(ctx, width=16, height=8, batch=2):
@@ -106,4 +106,17 @@ def test_noalloc_reports_its_own_errors(fake):  # noqa: F811
         assert fake.lf_render_noalloc(scene.h, C.byref(p), 0, 1, d) == 0
         assert ctx.device_errors() == 1
         ctx._c(fake.lf_device_free(ctx.h, d))
+        scene.close()
+
+
+def test_a_failed_allocation_is_reported_once(fake):  # noqa: F811
+    with lf.Context(0) as ctx:
+        scene, f = _frame(ctx)
+        f.render(0, 1)
+        fake.fake_fail_alloc(0)
+        with pytest.raises(lf.LFError) as err:
+            f.render(0, 1)
+        assert err.value.status == 3
+        f.render(0, 1)   # its launches do not find the earlier call's error
+        f.close()
         scene.close()
