@@ -1398,6 +1398,28 @@ cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb)
     const size_t bytes = n * 3 * sizeof(float);
     float* packed = nullptr;
     cudaError_t e = cudaMallocAsync((void**)&packed, bytes, st);
+    if (e == cudaErrorMemoryAllocation)
+    {
+        // a finished image can be read on a full device too: padded, in pieces, repacked here
+        cudaGetLastError();
+        constexpr size_t kPiece = 1 << 16;
+        std::vector<float4> tmp(std::min(n, kPiece));
+        for (size_t at = 0; at < n; at += kPiece)
+        {
+            const size_t m = std::min(n - at, kPiece);
+            e = cudaMemcpyAsync(tmp.data(), src + at, m * sizeof(float4), cudaMemcpyDeviceToHost, st);
+            const cudaError_t s = cudaStreamSynchronize(st);
+            if (e == cudaSuccess) e = s;
+            if (e != cudaSuccess) return e;
+            for (size_t k = 0; k < m; ++k)
+            {
+                rgb[3 * (at + k) + 0] = tmp[k].x;
+                rgb[3 * (at + k) + 1] = tmp[k].y;
+                rgb[3 * (at + k) + 2] = tmp[k].z;
+            }
+        }
+        return e;
+    }
     if (e != cudaSuccess) return e;
     e = (cudaError_t)launch_pack_rgb(src, (long long)n, packed, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(rgb, packed, bytes, cudaMemcpyDeviceToHost, st);

@@ -120,3 +120,18 @@ def test_a_failed_allocation_is_reported_once(fake):  # noqa: F811
         f.render(0, 1)   # its launches do not find the earlier call's error
         f.close()
         scene.close()
+
+
+@pytest.mark.parametrize("width,height", [(13, 7), (256, 256), (256, 257)])   # 2^16 pixels are one piece
+def test_readback_without_device_memory(fake, width, height):  # noqa: F811
+    """A rendered image can be read when nothing is left to allocate on the device."""
+    n = width * height
+    a = np.arange(4 * n, dtype=np.float32)
+    with lf.Context(0) as ctx:
+        scene, f = _frame(ctx, width, height)
+        ctx.sync()
+        C.memmove(fake.fake_block(16 * n, POOL), a.ctypes.data, a.nbytes)
+        fake.fake_fail_alloc(0)
+        assert np.array_equal(f.accum().reshape(-1, 3), a.reshape(-1, 4)[:, :3])
+        f.close()
+        scene.close()
