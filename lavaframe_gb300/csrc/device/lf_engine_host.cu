@@ -359,7 +359,7 @@ lf_status frame_render_fitting(lf_frame* f, EngineHost* e, const Params& Pf, int
     const bool tiledFrames = (f->flags & LF_FRAME_TILED_FRAMES) != 0;
     const int tiles = f->numTilesX * f->numTilesY;
     float4* arena = nullptr;
-    cudaError_t err = cudaMallocAsync((void**)&arena, sizeof(float4) * (size_t)paths, c->stream);
+    cudaError_t err = pool_alloc(c, &arena, sizeof(float4) * (size_t)paths, c->stream);
     if (err != cudaSuccess) return cuda_fail(c, err, "pass radiance allocation");
     std::vector<EnginePass> run;
     unsigned long long base = 0;
@@ -436,7 +436,7 @@ lf_status frame_render_fitting(lf_frame* f, EngineHost* e, const Params& Pf, int
         if (run.size() > 1)
         {
             const size_t bytes = sizeof(float4) * (size_t)last.numPaths;
-            err = cudaMallocAsync((void**)&copy, bytes, c->stream);
+            err = pool_alloc(c, &copy, bytes, c->stream);
             if (err != cudaSuccess)
             {
                 cudaGetLastError();
@@ -536,7 +536,7 @@ lf_status frame_render_engine(lf_frame* f, const Params& Pf, int firstSample, in
                     st = flush();
                     if (st != LF_OK) return st;
                 }
-                cudaError_t err = cudaMallocAsync((void**)&q.radiance, bytes, c->stream);
+                cudaError_t err = pool_alloc(c, &q.radiance, bytes, c->stream);
                 if (err != cudaSuccess) return cuda_fail(c, err, "pass radiance allocation");
                 engine_pass_submit(e, q);
                 run.push_back({q});

@@ -27,6 +27,7 @@ struct lf_ctx
 {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaMemPool_t pool = nullptr;   // stream-ordered memory (pool_acquire)
     std::recursive_mutex mu;
     std::string err;
     // status words of the kernels ([0]; [1] for lf_render_noalloc, which reports its own): in mapped page-locked memory, so that reading it after a
@@ -172,6 +173,14 @@ inline cudaError_t dalloc(std::vector<void*>& list, size_t& bytes, T** p, size_t
     return e;
 }
 
+// Stream-ordered memory of the library's own pool of the context's device (given back with
+// cudaFreeAsync).
+template <class T>
+inline cudaError_t pool_alloc(const lf_ctx* c, T** p, size_t bytes, cudaStream_t st)
+{
+    return cudaMallocFromPoolAsync((void**)p, bytes, c->pool, st);
+}
+
 inline lf_status check_device(lf_ctx* c)
 {
     cudaError_t e = cudaStreamSynchronize(c->stream);
@@ -219,8 +228,8 @@ constexpr size_t kStageBytes = size_t(1) << 18;
 bool ensure_stage(lf_ctx* c);
 // The copy streams and events of calls that overlap copies with kernels, made on first use.
 cudaError_t ensure_chunk_streams(lf_ctx* c);
-// The colour channels of n padded pixels into host memory, after the stream's work (synchronises).
-cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb);
+// The colour channels of n padded pixels into host memory, after the work of `st` (synchronises).
+cudaError_t copy_rgb(const lf_ctx* c, cudaStream_t st, const float4* src, size_t n, float* rgb);
 
 struct RefNode
 {

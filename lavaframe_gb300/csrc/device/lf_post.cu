@@ -200,8 +200,8 @@ extern "C" lf_status lf_frame_postprocess(lf_frame* f, const lf_post_params* pp,
     uint8_t* d8 = direct8 ? rgb8 : nullptr;
     float* df = directf ? rgbf : nullptr;
     cudaError_t e = cudaSuccess;
-    if (rgb8 && !direct8) e = cudaMallocAsync((void**)&d8, pix * 3, c->stream);
-    if (e == cudaSuccess && rgbf && !directf) e = cudaMallocAsync((void**)&df, pix * 3 * sizeof(float), c->stream);
+    if (rgb8 && !direct8) e = pool_alloc(c, &d8, pix * 3, c->stream);
+    if (e == cudaSuccess && rgbf && !directf) e = pool_alloc(c, &df, pix * 3 * sizeof(float), c->stream);
     if (e != cudaSuccess)
     {
         if (d8 && !direct8) cudaFreeAsync(d8, c->stream);

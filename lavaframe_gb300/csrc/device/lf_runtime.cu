@@ -3,10 +3,11 @@
 // render targets. Host code here must be compiled with -ffp-contract=off: light
 // precomputation and matrix inverses are part of the arithmetic contract.
 #include <algorithm>
-#include <limits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -19,6 +20,54 @@
 #include "lf_pixel.h"
 
 using namespace lfrt;
+
+namespace
+{
+// Frame buffers, pass radiance and job images come from a stream-ordered pool of the library, one per
+// device, made by the first context there and destroyed with the last. It keeps up to 8 GB between
+// calls instead of handing them back to CUDA at every synchronisation. (The device's default
+// pool is shared with whoever else allocates in the process; its threshold is theirs.)
+struct DevicePool
+{
+    cudaMemPool_t pool = nullptr;
+    int users = 0;
+};
+std::mutex g_pool_mu;
+std::map<int, DevicePool> g_pools;
+
+cudaError_t pool_acquire(int device, cudaMemPool_t* out)
+{
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevicePool& d = g_pools[device];
+    if (!d.pool)
+    {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        const cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
+        if (e != cudaSuccess)
+        {
+            d.pool = nullptr;
+            return e;
+        }
+        uint64_t keep = uint64_t(8) << 30;
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    ++d.users;
+    *out = d.pool;
+    return cudaSuccess;
+}
+
+void pool_release(int device)
+{
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevicePool& d = g_pools[device];
+    if (--d.users > 0) return;
+    cudaMemPoolDestroy(d.pool);   // blocks still allocated keep it until they are freed
+    d = DevicePool{};
+}
+}
 
 extern "C" {
 
@@ -35,7 +84,8 @@ lf_status lf_ctx_create(int32_t device, lf_ctx** out)
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaHostAlloc((void**)&c->h_status, 2 * sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
         (e = cudaHostGetDevicePointer((void**)&c->d_status, (void*)c->h_status, 0)) != cudaSuccess ||
-        (e = cudaMalloc((void**)&c->d_stats, 3 * sizeof(unsigned long long))) != cudaSuccess)
+        (e = cudaMalloc((void**)&c->d_stats, 3 * sizeof(unsigned long long))) != cudaSuccess ||
+        (e = pool_acquire(device, &c->pool)) != cudaSuccess)
     {
         delete c;
         return e == cudaErrorMemoryAllocation ? LF_ERR_OOM : LF_ERR_CUDA;
@@ -44,14 +94,6 @@ lf_status lf_ctx_create(int32_t device, lf_ctx** out)
     int coherent = 0;
     if (cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) == cudaSuccess)
         c->hostDirect = coherent != 0;
-    // frame buffers and pass radiance come from the stream-ordered pool; keep up to 8 GB of it cached
-    // between calls instead of handing it back to CUDA at every synchronisation
-    cudaMemPool_t pool = nullptr;
-    if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess)
-    {
-        uint64_t keep = uint64_t(8) << 30;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
     cudaMemset(c->d_stats, 0, 3 * sizeof(unsigned long long));
     *out = c;
     return LF_OK;
@@ -64,6 +106,7 @@ void lf_ctx_destroy(lf_ctx* c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     engine_destroy(c->engine);
     c->engine = nullptr;
+    if (c->pool) pool_release(c->device);
     cudaFreeHost((void*)c->h_status);
     cudaFreeHost(c->stage);
     cudaFree(c->d_stats);
@@ -1393,11 +1436,11 @@ bool direct_host(const lf_ctx* c, const void* p, size_t bytes, bool write, size_
 // The three colour channels of n padded pixels in the caller's buffer: packed on the device and
 // copied there directly (copying the padded pixels for the host to repack took 2.4 ms more of a
 // 1920 x 1080 x 16 render: 30.7 -> 28.3 ms).
-cudaError_t copy_rgb(cudaStream_t st, const float4* src, size_t n, float* rgb)
+cudaError_t copy_rgb(const lf_ctx* c, cudaStream_t st, const float4* src, size_t n, float* rgb)
 {
     const size_t bytes = n * 3 * sizeof(float);
     float* packed = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&packed, bytes, st);
+    cudaError_t e = pool_alloc(c, &packed, bytes, st);
     if (e == cudaErrorMemoryAllocation)
     {
         // a finished image can be read on a full device too: padded, in pieces, repacked here
@@ -1531,7 +1574,7 @@ lf_status lf_frame_create(lf_ctx* c, lf_scene* sc, const lf_render_params* p, ui
     unsigned long long* ctr = nullptr;
     // from the stream-ordered pool, so that making and releasing frames does not map memory
     auto A = [&](auto** p, size_t n) {
-        cudaError_t err = cudaMallocAsync((void**)p, sizeof(**p) * n, c->stream);
+        cudaError_t err = pool_alloc(c, p, sizeof(**p) * n, c->stream);
         if (err == cudaSuccess) f->fixedAllocs.push_back(*p);
         return err;
     };
@@ -1824,7 +1867,7 @@ lf_status lf_frame_read_accum(lf_frame* f, float* rgb)
     lf_ctx* c = f->ctx;
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     cudaSetDevice(c->device);
-    const cudaError_t e = copy_rgb(c->stream, f->accum, (size_t)f->W * f->H, rgb);
+    const cudaError_t e = copy_rgb(c, c->stream, f->accum, (size_t)f->W * f->H, rgb);
     if (e != cudaSuccess) return cuda_fail(c, e, "accum readback");
     return check_device(c);
 }

@@ -177,7 +177,7 @@ bool admit(lf_server* s, ServerJob& j)
     j.engineJob = engine_job_alloc(s->engine, sc.dev->view, j.P);
     if (j.engineJob < 0) return false;
     j.accumBytes = (size_t)j.params.width * j.params.height * sizeof(float4);
-    if (cudaMallocAsync((void**)&j.accum, j.accumBytes, c->stream) != cudaSuccess)
+    if (pool_alloc(c, &j.accum, j.accumBytes, c->stream) != cudaSuccess)
     {
         cudaGetLastError();
         engine_job_free(s->engine, j.engineJob);
@@ -211,7 +211,7 @@ bool issue_passes(lf_server* s, ServerJob& j)
         q.visH = j.params.height;
         q.numPaths = (unsigned long long)n * q.visW * q.visH;
         sp.bytes = sizeof(float4) * q.numPaths;   // within the job's reservation
-        if (cudaMallocAsync((void**)&q.radiance, sp.bytes, c->stream) != cudaSuccess)
+        if (pool_alloc(c, &q.radiance, sp.bytes, c->stream) != cudaSuccess)
         {
             cudaGetLastError();
             break;
@@ -521,7 +521,7 @@ lf_status lf_server_read(lf_server* s, int64_t job_id, float* rgb)
     cudaSetDevice(c->device);
     // a done job's image is complete (its event has passed), so it is read on a stream of its own, beside
     // the step pair that the scheduler has in flight
-    const cudaError_t e = copy_rgb(s->readStream, j.accum, (size_t)j.params.width * j.params.height, rgb);
+    const cudaError_t e = copy_rgb(c, s->readStream, j.accum, (size_t)j.params.width * j.params.height, rgb);
     if (e == cudaSuccess) return LF_OK;
     std::lock_guard<std::recursive_mutex> g(c->mu);
     return cuda_fail(c, e, "job readback");

@@ -135,3 +135,17 @@ def test_readback_without_device_memory(fake, width, height):  # noqa: F811
         assert np.array_equal(f.accum().reshape(-1, 3), a.reshape(-1, 4)[:, :3])
         f.close()
         scene.close()
+
+
+def test_the_default_memory_pool_is_left_alone(fake):  # noqa: F811
+    """Contexts of a device share a pool of the library's own, which goes with the last of them."""
+    with lf.Context(0) as a, lf.Context(0) as b:
+        for ctx in (a, b):
+            scene, f = _frame(ctx)
+            f.render(0, 5)
+            f.accum()
+            assert fake.fake_pool_blocks(0) > 0 and fake.fake_pool_blocks(1) == 0
+            f.close()
+            scene.close()
+        assert fake.fake_pools() == 1
+    assert fake.fake_pools() == 0 and fake.fake_default_pool_changes() == 0
