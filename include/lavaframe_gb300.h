@@ -212,7 +212,9 @@ typedef struct lf_hit
  * input order (closest hits on scenes of more than 1.5M triangles from 2^19 rays up are
  * binned instead). Otherwise: copies rays in, traces, copies hits out; when the output lies in one
  * block from lf_host_alloc of this context, the kernels write the results there and nothing
- * is copied back. */
+ * is copied back. A call that ends in LF_ERR_DEVICE returns the results of every ray that had no
+ * error; after any other error the result buffer's contents are undefined, as kernels may have
+ * written a part of it. */
 lf_status lf_trace_closest(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, lf_hit* hits, uint32_t flags);
 /* occluded[i] = 1 when something lies closer than tmax. */
 lf_status lf_trace_any(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, uint8_t* occluded, uint32_t flags);

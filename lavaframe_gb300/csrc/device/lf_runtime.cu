@@ -1316,8 +1316,9 @@ lf_status trace_host(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, void
         std::memcpy(c->stage, rays, (size_t)n * 32);
         lf_status sst = launch(c->d_stage, c->d_stage + (size_t)n * 32, n, 0);
         const lf_status dst = check_device(c);
+        // an error bit ends single rays: the others' results are good
+        if (sst == LF_OK && (dst == LF_OK || dst == LF_ERR_DEVICE)) std::memcpy(out, s_out, (size_t)n * outElem);
         if (sst == LF_OK) sst = dst;
-        if (sst == LF_OK) std::memcpy(out, s_out, (size_t)n * outElem);
         if (sst == LF_OK && (flags & LF_TRACE_STATS)) read_trace_stats(c);
         return sst;
     }

@@ -149,3 +149,29 @@ def test_the_default_memory_pool_is_left_alone(fake):  # noqa: F811
             scene.close()
         assert fake.fake_pools() == 1
     assert fake.fake_pools() == 0 and fake.fake_default_pool_changes() == 0
+
+
+@pytest.mark.parametrize("n", [100, 20000])   # over the staging block and over copies
+def test_results_beside_a_device_error(fake, n):  # noqa: F811
+    """An error bit of one ray's traversal leaves the other rays' results: they are returned with the
+    error, whatever way they came."""
+    want = np.arange(4 * n, dtype=np.int32)
+    with lf.Context(0) as ctx:
+        scene, f = _frame(ctx)
+        status = C.cast(fake.fake_block(8, PINNED), C.POINTER(C.c_uint32))
+
+        def launched(name, args):
+            if b"trace_fetch_wide" in name:
+                fake.fake_flush()
+                C.memmove(C.cast(args[4], C.POINTER(C.c_void_p))[0], want.ctypes.data, want.nbytes)
+                status[0] = 1
+
+        hook = HOOK(launched)
+        fake.fake_hook(hook)
+        rays, out = np.zeros((n, 8), np.float32), np.zeros((n, 4), np.int32)
+        st = fake.lf_trace_closest(ctx.h, scene.h, rays.ctypes.data_as(C.POINTER(C.c_float)), n,
+                                   out.ctypes.data_as(C.c_void_p), 0)
+        fake.fake_hook(HOOK())
+        assert st == 4 and ctx.device_errors() == 1 and out.reshape(-1).tobytes() == want.tobytes()
+        f.close()
+        scene.close()
