@@ -210,7 +210,6 @@ __global__ void engine_init_kernel(EngineBuffers b)
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         b.ctl->freeCount = b.cap;
-        b.ctl->taken = 0;
         b.ctl->doneCount[0] = 0;
         b.ctl->doneCount[1] = 0;
         b.ctl->active = 0;

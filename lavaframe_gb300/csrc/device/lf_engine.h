@@ -67,7 +67,6 @@ struct EngineCtl
     int doneCount[2];              // done-list sizes
     int active;                    // paths started and not yet written out
     int freeCount;                 // free slots (info.w == -1)
-    int taken;                     // slots the current step's refill started
     int extendNext, shadeNext, shadowNext;   // work counters of the extend, shade and shadow kernels
     int refillNext;                // ids handed out by the current refill
     int refillDone, shadowDone;    // blocks that have ended (the last one resets the step's counters)

@@ -226,8 +226,6 @@ inline bool disjoint(const void* a, size_t na, const void* b, size_t nb)
 // false when there is none.
 constexpr size_t kStageBytes = size_t(1) << 18;
 bool ensure_stage(lf_ctx* c);
-// The copy streams and events of calls that overlap copies with kernels, made on first use.
-cudaError_t ensure_chunk_streams(lf_ctx* c);
 // The colour channels of n padded pixels into host memory, after the work of `st` (synchronises).
 cudaError_t copy_rgb(const lf_ctx* c, cudaStream_t st, const float4* src, size_t n, float* rgb);
 

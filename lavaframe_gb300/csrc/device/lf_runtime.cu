@@ -1109,7 +1109,11 @@ bool ensure_stage(lf_ctx* c)
     }
     return true;
 }
+}
 
+namespace
+{
+// The copy streams and events of host queries in several pieces, made on first use.
 cudaError_t ensure_chunk_streams(lf_ctx* c)
 {
     if (c->copyOut) return cudaSuccess;
@@ -1124,10 +1128,7 @@ cudaError_t ensure_chunk_streams(lf_ctx* c)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->chunkEnd, cudaEventDisableTiming);
     return e;
 }
-}
 
-namespace
-{
 // Scratch of the ray queries: the fetch counters, and for a binned query of n rays the bins, keys
 // and permutation.
 lf_status ensure_bin_scratch(lf_ctx* c, long long n, bool binned)
@@ -2060,7 +2061,8 @@ constexpr size_t kNoAllocAlign = 256;
 constexpr size_t kNoAllocHeader = 1024;       // control block, pass, counters
 constexpr size_t noalloc_round(size_t b) { return (b + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
 // PathSoA: o, d, T, L, A, rng, info, hit and the radiance (16 B each), luv (8 B); two queues and the
-// split one (4 B each); next-event records
+// split one (4 B each); next-event records. (A run is one launch, which needs neither L nor queues nor
+// records, unless its depth is above kThreadBounces.)
 constexpr size_t kNoAllocBytes = kNoAllocHeader + 9 * noalloc_round(kNoAllocPaths * 16) +
                                  noalloc_round(kNoAllocPaths * 8) + 3 * noalloc_round(kNoAllocPaths * 4) +
                                  noalloc_round(kNoAllocPaths * sizeof(ShadowRec));
