@@ -711,19 +711,20 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     const bool directIn = direct_host(c, samples, (size_t)n * kSampleFloats * sizeof(float), false);
     const bool directGrid = disjoint(samples, (size_t)n * kSampleFloats * sizeof(float), dgrid, gridBytes) &&
                             direct_host(c, dgrid, gridBytes, true);
-    lf_status st = ensure_scratch(gd, (directIn ? 0 : (size_t)n * kSampleFloats) + (directGrid ? 0 : kGridParams));
-    if (st != LF_OK) return st;
-    if (!ensure_stage(c)) return fail(c, LF_ERR_OOM, "guide gradient staging");
-    float* const outGrid = directGrid ? dgrid : gd->scratch;
-    const float* in = samples;
-    // the small results go to page-locked memory, which saves two copies' latencies
+    // the small results go to page-locked memory, which saves two copies' latencies, if there is some
     static_assert((kWeights + 1) * sizeof(float) <= kStageBytes, "weight gradients and the loss fit the staging block");
-    float* const hW = reinterpret_cast<float*>(c->stage);
-    float* const dW = reinterpret_cast<float*>(c->d_stage);
+    const bool staged = ensure_stage(c);
+    // scratch: grid gradients, samples, weight gradients and loss, each 16-byte aligned
+    const size_t gf = directGrid ? 0 : kGridParams, sf = directIn ? 0 : (size_t)n * kSampleFloats;
+    lf_status st = ensure_scratch(gd, gf + sf + (staged ? 0 : kWeights + 1));
+    if (st != LF_OK) return st;
+    float* const outGrid = directGrid ? dgrid : gd->scratch;
+    float* const dW = staged ? reinterpret_cast<float*>(c->d_stage) : gd->scratch + gf + sf;
+    const float* in = samples;
     if (!directIn)
     {
-        float* const copy = gd->scratch + (directGrid ? 0 : kGridParams);   // 16-byte aligned
-        cudaMemcpyAsync(copy, samples, (size_t)n * kSampleFloats * sizeof(float), cudaMemcpyHostToDevice, c->stream);
+        float* const copy = gd->scratch + gf;
+        cudaMemcpyAsync(copy, samples, sf * sizeof(float), cudaMemcpyHostToDevice, c->stream);
         in = copy;
     }
     cudaMemsetAsync(gd->dLoss, 0, sizeof(double), c->stream);      // training steps leave theirs
@@ -736,10 +737,19 @@ lf_status lf_guide_gradients(lf_guide* gd, const float* samples, int32_t n, floa
     guide_scale_kernel<<<(kWeights + kGridParams) / 4 / 256 + 1, 256, 0, c->stream>>>(
         gd->wGrad, gd->gGrad, gd->dLoss, 1.f / (float)n, dW, outGrid, dW + kWeights);
     if (!directGrid) cudaMemcpyAsync(dgrid, outGrid, gridBytes, cudaMemcpyDeviceToHost, c->stream);
+    if (!staged)
+    {
+        cudaMemcpyAsync(dweights, dW, kWeights * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+        cudaMemcpyAsync(loss, dW + kWeights, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    }
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "guide gradients");
-    std::memcpy(dweights, hW, kWeights * sizeof(float));
-    *loss = hW[kWeights];
+    if (staged)
+    {
+        const float* const hW = reinterpret_cast<const float*>(c->stage);
+        std::memcpy(dweights, hW, kWeights * sizeof(float));
+        *loss = hW[kWeights];
+    }
     return check_device(c);
 }
 

@@ -35,7 +35,7 @@ std::deque<Op> queue;
 std::map<char*, Block> blocks;
 std::map<const void*, std::string> kernels;
 std::map<const void*, std::pair<void*, size_t>> vars;
-int badFrees = 0, changedSources = 0, failAlloc = -1, failLaunch = -1, coherent = 0;
+int badFrees = 0, changedSources = 0, failAlloc = -1, failKind = -1, failLaunch = -1, coherent = 0;
 cudaError_t lastError = cudaSuccess;
 int defaultPool, defaultPoolChanges = 0, pools = 0;
 void (*hook)(const char*, void**) = nullptr;
@@ -82,6 +82,7 @@ cudaError_t done(cudaError_t e)
 cudaError_t alloc(void** p, size_t bytes, int kind, cudaMemPool_t pool)
 {
     Lock l(mu);
+    if (kind == failKind) return done(cudaErrorMemoryAllocation);
     if (failAlloc >= 0 && failAlloc-- == 0) return done(cudaErrorMemoryAllocation);   // *p stays as it was
     *p = std::calloc(bytes ? bytes : 1, 1);
     blocks[(char*)*p] = {bytes ? bytes : 1, kind, pool};
@@ -120,7 +121,7 @@ void fake_reset()
     Lock l(mu);
     flush();
     badFrees = changedSources = defaultPoolChanges = 0;
-    failAlloc = failLaunch = -1;
+    failAlloc = failKind = failLaunch = -1;
     lastError = cudaSuccess;
     hook = nullptr;
     coherent = 0;
@@ -131,6 +132,7 @@ void fake_flush()
     flush();
 }
 void fake_fail_alloc(int after) { failAlloc = after; }     // the allocation that `after` others precede
+void fake_fail_alloc_kind(int kind) { failKind = kind; }   // all allocations of this kind
 void fake_fail_launch(int after) { failLaunch = after; }
 // called for every launch with the kernel's name and the addresses of its arguments
 void fake_hook(void (*f)(const char*, void**)) { hook = f; }

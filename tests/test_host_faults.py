@@ -175,3 +175,32 @@ def test_results_beside_a_device_error(fake, n):  # noqa: F811
         assert st == 4 and ctx.device_errors() == 1 and out.reshape(-1).tobytes() == want.tobytes()
         f.close()
         scene.close()
+
+
+@pytest.mark.parametrize("coherent", [0, 1])
+@pytest.mark.parametrize("locked", [True, False])
+def test_gradients_without_page_locked_memory(fake, locked, coherent):  # noqa: F811
+    """The small results of a gradient call go over page-locked memory if there is some."""
+    n, nW = 200, lf.GUIDE_WEIGHTS
+    want = np.arange(nW + 1, dtype=np.float32)
+    grid = np.arange(lf.GUIDE_GRID_PARAMS, dtype=np.float32)
+    fake.fake_coherent(coherent)
+    with lf.Context(0) as ctx:
+        g = lf.Guide(ctx, [0, 0, 0], [1, 1, 1], seed=3)
+
+        def launched(name, args):
+            if b"guide_scale_kernel" in name:
+                fake.fake_flush()
+                at = [C.cast(args[k], C.POINTER(C.c_void_p))[0] for k in (4, 5, 6)]
+                C.memmove(at[0], want.ctypes.data, 4 * nW)
+                C.memmove(at[1], grid.ctypes.data, grid.nbytes)
+                C.memmove(at[2], want.ctypes.data + 4 * nW, 4)
+
+        hook = HOOK(launched)
+        fake.fake_hook(hook)
+        if not locked:
+            fake.fake_fail_alloc_kind(PINNED)
+        loss, dw, dg = g.gradients(np.zeros((n, 16), np.float32))
+        fake.fake_hook(HOOK())
+        assert dw.tobytes() == want[:nW].tobytes() and dg.tobytes() == grid.tobytes() and loss == nW
+        g.close()
