@@ -624,13 +624,19 @@ lf_status encode_wide(lf_ctx* c, const lf_scene_view* v, const RefNode* nodes, s
         }
     }
     // instances merged into the instance level: identity inverse (bit for bit), a mesh of their own
-    std::vector<unsigned char> shared(v->num_nodes, 0);
-    mark_shared(B, instRoot, shared);
     const float4 identity[3] = {make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0), make_float4(1, 0, 0, 0)};
+    std::vector<int> merged;
     for (int i = 0; i < v->num_instances; ++i)
         if (instRoot[i] >= 0 && instRoot[i] < v->num_nodes && rootUses[instRoot[i]] == 1 &&
-            !shared[instRoot[i]] && std::memcmp(&inst[(size_t)i * 4], identity, sizeof identity) == 0 && inlinable(B, instLeaf[i], instRoot[i]))
-            B.inlineRoot[i] = instRoot[i];
+            std::memcmp(&inst[(size_t)i * 4], identity, sizeof identity) == 0 && inlinable(B, instLeaf[i], instRoot[i]))
+            merged.push_back(i);
+    if (!merged.empty())
+    {
+        std::vector<unsigned char> shared(v->num_nodes, 0);
+        mark_shared(B, instRoot, shared);
+        for (const int i : merged)
+            if (!shared[instRoot[i]]) B.inlineRoot[i] = instRoot[i];
+    }
     for (int i = 0; i < v->num_instances; ++i)
     {
         int code = ~0, rootRef = -1;
