@@ -219,8 +219,9 @@ lf_status lf_trace_closest(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n
 /* occluded[i] = 1 when something lies closer than tmax. */
 lf_status lf_trace_any(lf_ctx* c, lf_scene* sc, const float* rays, int64_t n, uint8_t* occluded, uint32_t flags);
 /* Host-buffer queries split the rays into `chunks` pieces (1..8; 0 = automatic, the
- * default: two pieces from 2^24 rays up, else one; more than one always go over copies): piece k+1 is copied in and piece k-1
- * copied out while piece k is sorted and traced. Every ray's result is the same for any
+ * default: queries that are not traced in place go in two pieces from 2^24 rays up, else in one;
+ * a setting above 1 takes every query over copies): piece k+1 is copied in and piece k-1 copied
+ * out while piece k is sorted and traced. Every ray's result is the same for any
  * setting; LF_TRACE_STATS queries run whole. */
 lf_status lf_ctx_set_host_chunks(lf_ctx* c, int32_t chunks);
 /* Device buffers, asynchronous on the context stream (lf_ctx_sync to wait). */

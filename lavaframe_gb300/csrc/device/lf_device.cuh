@@ -217,9 +217,9 @@ __device__ __forceinline__ float xor_sign(float a, float b)
 // determinant decide what the quotients' tests would, and only triangles met close to an edge form
 // them (the same IEEE divisions as in tri_hit). Rejected: u or v below zero by more than the
 // smallest quotient that rounds to a negative number (|det| 1e-30), or u or u + v above |det| by more
-// than the rounding of the sums. Accepted: the same margins inside. A determinant that is zero,
-// infinite or NaN fails every comparison (or accepts nothing) and leaves the decision to the
-// quotients; the distance is always tri_hit's quotient. Leaf visits are bound by instruction issue
+// than the rounding of the sums. Accepted: the same margins inside. Of a zero determinant both margins
+// are zero: any numerator that is not zero is rejected, as its quotient's infinity is; an infinite or NaN
+// one fails the comparisons or leaves the decision to the quotients; the distance is always tri_hit's quotient. Leaf visits are bound by instruction issue
 // with two or three lanes active, so what counts is how early all of them are done: 4M rays against
 // 1.3M random triangles 4.97 -> 4.61 ms, occlusion 4.47 -> 4.00, 2M rays on spheres 677 -> 641 and
 // 552 -> 506 us, in a room 505 -> 500 and 248 -> 238, spheres 1080p x 8 13.9 -> 13.3 ms. (Without the

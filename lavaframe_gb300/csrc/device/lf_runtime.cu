@@ -1280,8 +1280,8 @@ void read_trace_stats(lf_ctx* c)
 // (1M closest hits on the Cornell box 0.65 against 0.48 ms), so those work on copies. Direct in
 // input order / copied and binned, us, on the Cornell box, a room, spheres, 1.3M, 2M and 5.2M random
 // triangles: 600k rays 167 / 317, 227 / 367, 254 / 418, 984 / 999, 1082 / 1039, 1415 / 1326; 4M rays
-// 799 / 1676, 1193 / 1996, 1263 / 2184, 5413 / 5576, 5968 / 5757, 8100 / 6971. Binning pays once
-// triangles and nodes outgrow the 129 MB L2. Occlusion, 12M rays: 10.6 / 11.7 ms on 2M triangles,
+// 799 / 1676, 1193 / 1996, 1263 / 2184, 5413 / 5576, 5968 / 5757, 8100 / 6971. Binning with its copies
+// pays on scenes well beyond the 129 MB L2, between 1.3M and 2M triangles. Occlusion, 12M rays: 10.6 / 11.7 ms on 2M triangles,
 // 11.8 / 12.2 on 5.2M; equal on 10.5M. Sizes that are not binned either way: 8,000 closest hits 53 ->
 // 31 us, 300,000 179 -> 104.
 constexpr int kDirectClosestTris = 1500000;

@@ -34,9 +34,10 @@ static_assert(kScanBlocks >= 1 && kScanBlocks <= 2 * kScanBlock, "bin scan cover
 // Up to 1.2M (Cornell 35k, room 48k, spheres 164k, random 327k): 524k rays 141 / 135, 169 / 175, 186 / 168,
 // 624 / 636, 800k 189 / 189, 230 / 245, 243 / 225, 889 / 907, 2^21 415 / 446, 517 / 585, 512 / 504,
 // 2148 / 2217: 2^19 lies between them (3 * 2^18 gives spheres 16 % there and takes 5 % from the
-// room). Beyond the L2 (1.3M, 2M, 5.2M random triangles): 131k 283 / 274, -, 407 / 401, 262k 445 / 492,
-// 495 / 534, 643 / 671, 524k 751 / 835, 779 / 935, 1047 / 1212. Queries of host buffers have a rule of
-// their own (direct_query).
+// room). Scenes larger than the L2 (1.3M, 2M, 5.2M random triangles, about 200 bytes each): 131k
+// 283 / 274, -, 407 / 401, 262k 445 / 492, 495 / 534, 643 / 671, 524k 751 / 835, 779 / 935, 1047 / 1212. The
+// lines are triangle counts between measured scenes; nothing between 327k and 1.3M was measured. Queries
+// of host buffers have a rule of their own (direct_query), as their binning also costs the copies.
 long long sort_closest(int tris)
 {
     if (tris <= 1 << 13) return 1 << 21;
